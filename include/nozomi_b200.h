@@ -449,6 +449,12 @@ int nz_moments(const float* spins, const float* spins0, int N, double* out, void
  * divides its FP32 work by this peak. ---- */
 int nz_probe_fma(int grid, int iters, float* out, void* stream);
 
+/* ---- testing aid (no reference counterpart): the Box-Muller transform of
+ * the walks' draws on given words: words [n][4] (a0, b0, a1, b1), out [n][4]
+ * (the cosine and sine normals of (a0, b0), then of (a1, b1)), both 16-byte
+ * aligned. ---- */
+int nz_probe_box_muller(const uint32_t* words, int n, float* out, void* stream);
+
 #ifdef __cplusplus
 }
 #endif
