@@ -1,4 +1,5 @@
 // Seeding, walker re-binning, signal and moment reductions.
+#include <algorithm>
 #include <cstdint>
 #include <mutex>
 #include "kernels.cuh"
@@ -180,32 +181,63 @@ __device__ __forceinline__ double block_sum(double v, double* s_red) {
   return t;  // valid in thread 0
 }
 
-__global__ void __launch_bounds__(kSigThreads) signal_kernel(nz_state st, const float* __restrict__ dirs, int ndir,
-                                                             const float* __restrict__ amp, int nb,
-                                                             double* __restrict__ out) {
-  __shared__ double s_red[32];
-  const int w = blockIdx.x * blockDim.x + threadIdx.x;
-  float px = 0.f, py = 0.f, pz = 0.f;
-  const bool live = w < st.N;
-  if (live) {
-    const float4 f = reinterpret_cast<const float4*>(st.phi)[w];
-    const float4 c = reinterpret_cast<const float4*>(st.comp)[w];
-    px = f.x - c.x;
-    py = f.y - c.y;
-    pz = f.z - c.z;
+// A thread sums one (direction, b) over its share of the block's walkers, in
+// FP64 registers; the phase vectors of kSigTile walkers at a time wait in
+// shared memory.  `groups` threads share a (direction, b), each every
+// groups-th walker.  Bound by issue slots, nearly all of them
+// the sines' and cosines': 30 x 4 x 1e6 of them take 0.22 ms on a B200 (84 %
+// of the issue slots), 0.54 ms when every (direction, b) of 256 walkers was
+// summed over a block with two barriered reductions.
+constexpr int kSigTile = 512;
+constexpr int kSigMaxThreads = 384;
+
+__global__ void __launch_bounds__(kSigMaxThreads) signal_kernel(nz_state st, const float* __restrict__ dirs, int ndir,
+                                                                const float* __restrict__ amp, int nb, int combos,
+                                                                int groups, int per_block, double* __restrict__ out) {
+  __shared__ float4 s_p[kSigTile];
+  __shared__ double s_sum[2][kSigMaxThreads];
+  const int t = threadIdx.x, group = t / combos, combo = blockIdx.y * combos + t % combos;
+  const bool busy = group < groups && combo < ndir * nb;
+  float d0 = 0.f, d1 = 0.f, d2 = 0.f, a0 = 0.f;
+  if (busy) {
+    const int d = combo / nb;
+    d0 = dirs[d];
+    d1 = dirs[ndir + d];
+    d2 = dirs[2 * ndir + d];
+    a0 = amp[combo % nb];
   }
-  for (int d = 0; d < ndir; ++d) {
-    const float ph = px * __ldg(dirs + d) + py * __ldg(dirs + ndir + d) + pz * __ldg(dirs + 2 * ndir + d);
-    for (int b = 0; b < nb; ++b) {
-      float sn = 0.f, cs = 0.f;
-      if (live) sincosf(__ldg(amp + b) * ph, &sn, &cs);
-      const double re = block_sum(live ? double(cs) : 0.0, s_red);
-      const double im = block_sum(live ? double(sn) : 0.0, s_red);
-      if (threadIdx.x == 0) {
-        atomicAdd(out + d * nb + b, re);
-        atomicAdd(out + ndir * nb + d * nb + b, im);
-      }
+  double re = 0.0, im = 0.0;
+  const int first = blockIdx.x * per_block, last = min(st.N, first + per_block);
+  for (int base = first; base < last; base += kSigTile) {
+    const int n = min(kSigTile, last - base);
+    __syncthreads();
+    for (int i = t; i < n; i += blockDim.x) {
+      const float4 f = reinterpret_cast<const float4*>(st.phi)[base + i];
+      const float4 c = reinterpret_cast<const float4*>(st.comp)[base + i];
+      s_p[i] = make_float4(f.x - c.x, f.y - c.y, f.z - c.z, 0.f);
     }
+    __syncthreads();
+    if (!busy) continue;
+#pragma unroll 2
+    for (int i = group; i < n; i += groups) {
+      const float4 p = s_p[i];
+      const float ph = p.x * d0 + p.y * d1 + p.z * d2;
+      float sn, cs;
+      sincosf(a0 * ph, &sn, &cs);
+      re += double(cs);
+      im += double(sn);
+    }
+  }
+  s_sum[0][t] = re;
+  s_sum[1][t] = im;
+  __syncthreads();
+  if (t < combos && combo < ndir * nb) {
+    for (int g = 1; g < groups; ++g) {
+      re += s_sum[0][t + g * combos];
+      im += s_sum[1][t + g * combos];
+    }
+    atomicAdd(out + combo, re);
+    atomicAdd(out + ndir * nb + combo, im);
   }
 }
 
@@ -412,8 +444,26 @@ extern "C" int nz_signal_phi(const nz_state* st, const float* dirs, int ndir, co
   if (rc) return rc;
   if (!dirs || !amp || !out || ndir <= 0 || nb <= 0) return set_error(NZ_ERR_ARG, "nz_signal_phi: bad arguments");
   if (st->N == 0) return NZ_OK;
-  signal_kernel<<<(st->N + kSigThreads - 1) / kSigThreads, kSigThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-      *st, dirs, ndir, amp, nb, out);
+  // (direction, b) pairs of a block: all of them up to kSigMaxThreads, beyond
+  // that even shares; as many threads to each as leave the fewest idle.
+  const long long all = 1ll * ndir * nb;
+  if (all > 0x7fffffffll / 2) return set_error(NZ_ERR_ARG, "nz_signal_phi: %d directions x %d amplitudes", ndir, nb);
+  const int ny = int((all + kSigMaxThreads - 1) / kSigMaxThreads);
+  const int combos = int((all + ny - 1) / ny);
+  int groups = 1, threads = (combos + 31) / 32 * 32;
+  for (int g = 2; g * combos <= kSigMaxThreads; ++g) {
+    const int th = (g * combos + 31) / 32 * 32;
+    if (g * combos * threads >= groups * combos * th) {
+      groups = g;
+      threads = th;
+    }
+  }
+  // one wave of blocks (32 registers a thread: full SMs), each at least 64
+  // walkers
+  const int wave = std::max(1, 148 * (2048 / threads) / ny);
+  const int per_block = std::max(64, (st->N + wave - 1) / wave);
+  signal_kernel<<<dim3(unsigned((st->N + per_block - 1) / per_block), unsigned(ny)), threads, 0,
+                  static_cast<cudaStream_t>(stream)>>>(*st, dirs, ndir, amp, nb, combos, groups, per_block, out);
   return check_launch("signal_kernel");
 }
 
