@@ -80,21 +80,21 @@ KERNEL_SOURCES = ("nozomi_b200/csrc/walk_fused.cu", "nozomi_b200/csrc/nz_common.
 # dram__bytes_write.sum) of the captured launch, divided by the walker-steps
 # that launch ran; kernel_sha: the sources' hash at capture.
 PROFILED = {
-    "packed": {"kernel_sha": "e297eb0c11e140a9", "warp_inst_per_walker_step": 53.681,
-               "dram_bytes_per_walker_step": 0.9909,
+    "packed": {"kernel_sha": "90d5fe0fe07f3640", "warp_inst_per_walker_step": 53.673,
+               "dram_bytes_per_walker_step": 0.9890,
                "shape": {"cell": 0.5, "near_margin": 0.5, "coarsen": 8, "threads": 128, "lists": "index",
                          "near_shape": "round", "stage": 0},
                "capture": "walk_fused_kernel<PHI, idx16> launch 3 of `python bench.py --workload packed --walkers "
                           "1000000 --steps-per-launch 200 --steps 1 --warmup 1 --no-cpu-baseline --e2e-steps 0` "
-                          "(200,000,000 walker-steps): 10,736,161,297 warp instructions, 198.2 MB DRAM"},
-    "batched": {"kernel_sha": "e297eb0c11e140a9", "warp_inst_per_walker_step": 38.736,
-                "dram_bytes_per_walker_step": 0.2370,
+                          "(200,000,000 walker-steps): 10,734,677,185 warp instructions, 197.8 MB DRAM"},
+    "batched": {"kernel_sha": "90d5fe0fe07f3640", "warp_inst_per_walker_step": 38.734,
+                "dram_bytes_per_walker_step": 0.2387,
                 "shape": {"cell": 1.0, "near_margin": 0.5, "coarsen": 4, "threads": 256, "lists": "index",
                           "near_shape": "round", "stage": 0},
                 "capture": "walk_fused_kernel<PHI, idx16> launch 2 of `python bench.py --walker-scale 0.1 --steps 1 "
                            "--warmup 1 --no-serving --no-plain --no-cpu-baseline --e2e-steps 0 --no-autotune --cell 1.0 "
                            "--coarsen 4 --steps-per-launch 2000 --threads 256` (64 jobs, 2,407,477,000 walker-steps): "
-                           "93,255,911,087 warp instructions, 570.6 MB DRAM"},
+                           "93,252,190,386 warp instructions, 574.7 MB DRAM"},
 }
 
 

@@ -109,6 +109,13 @@ extern "C" int nz_walk_step(const nz_substrate* sub, const nz_walkers* wk, int m
   a.n_iter = wk->n_iter;
   a.n_scatter = wk->n_scatter;
   a.flags = wk->flags;
+  // index lists, where the substrate has them, hold the same members
+  if ((sub->idx_bytes == 2 || sub->idx_bytes == 4) && sub->cell_idx && sub->rec4 && sub->rec_sid && sub->sid_start &&
+      aligned16(sub->rec4) && (sub->idx_bytes == 4 || sub->S <= 65536))
+    return launch_plain_lists(a,
+                              PlainLists{sub->cell_idx, reinterpret_cast<const float4*>(sub->rec4), sub->rec_sid,
+                                         sub->sid_start},
+                              sub->idx_bytes, static_cast<cudaStream_t>(stream));
   walk_plain_kernel<<<(wk->N + 255) / 256, 256, 0, static_cast<cudaStream_t>(stream)>>>(a);
   return check_launch("walk_plain_kernel");
 }

@@ -46,6 +46,15 @@ struct PlainArgs {
   int* flags;
 };
 __global__ void walk_plain_kernel(const PlainArgs a);
+// Index lists of the plain walk (nz_substrate.idx_bytes): entries ascending
+// by record within a cell, records by structure.
+struct PlainLists {
+  const void* idx;
+  const float4* rec4;
+  const int* rec_sid;
+  const int* sid_start;
+};
+int launch_plain_lists(const PlainArgs& a, const PlainLists& l, int idx_bytes, cudaStream_t st);
 
 // ---- fused walk (walk_fused.cu) ----
 constexpr int kFusedThreads = 128;     // walkers per CTA of nz_walk_fused
