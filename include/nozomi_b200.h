@@ -263,7 +263,8 @@ int nz_ingest_write(const double* rows, const int* ends, int F, const int* partn
  * Scratch shared by nz_collide_cells and the nz_collide_pairs that follows it. */
 size_t nz_collide_scratch_bytes(int S, const nz_grid* grid);
 /* Block ranges and member counts; *n_members (one device int) = the total
- * number of (block, sphere) memberships, the size of nz_collide_pairs' items. */
+ * number of (block, sphere) memberships, the size of nz_collide_pairs' items;
+ * -1 when a sphere's position or radius is not finite. */
 int nz_collide_cells(const float* pos, const float* radii, int S, const nz_grid* grid, int* n_members,
                      void* scratch, size_t scratch_bytes, void* stream);
 /* Every colliding pair, unordered, into pairs[cap][2]; *n_pairs = how many

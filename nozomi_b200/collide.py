@@ -48,8 +48,6 @@ def detect_collision(positions, radii, fiber_id, Lx, Ly, Lz, buff=0.0, sort: boo
     S = int(pos.shape[0])
     if r.numel() != S or fid.numel() != S:
         raise L.NozomiError("positions, radii and fiber_id need one row per sphere")
-    if S and not (torch.isfinite(pos).all() and torch.isfinite(r).all()):
-        raise L.NozomiError("sphere positions and radii must be finite")
     g = block_grid(float(Lx), float(Ly), float(Lz))
     stream = ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
     p = lambda t: ctypes.c_void_p(t.data_ptr())  # noqa: E731
@@ -59,6 +57,8 @@ def detect_collision(positions, radii, fiber_id, Lx, Ly, Lz, buff=0.0, sort: boo
     L.check(lib.nz_collide_cells(p(pos), p(r), S, ctypes.byref(g), p(counts), p(scratch), scratch.numel(), stream),
             "nz_collide_cells")
     members = int(counts[0].item())
+    if members < 0:
+        raise L.NozomiError("sphere positions and radii must be finite")
     items = torch.empty(max(members, 1), dtype=torch.int32, device=dev)
     cap = max(1024, 4 * S)
     for _ in range(2):  # a second pass only when the first buffer was too small

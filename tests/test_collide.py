@@ -81,3 +81,53 @@ def test_block_grid_is_the_reference_grid():
         n, d, _ = oracle_grid(*L)
         assert (g.nx, g.ny, g.nz) == tuple(int(v) for v in n)
         assert np.array([g.dLx, g.dLy, g.dLz], np.float32).tobytes() == d.tobytes()
+
+
+def _crowd(S, L, seed, rmax):
+    """S spheres anywhere in a box so small that each block lists most of
+    them (or, in a long box, few); seed chosen so that no pair's distance is
+    within 1e-6 um of its threshold, far above float32 rounding."""
+    rng = np.random.default_rng(seed)
+    pos = (rng.uniform(-0.5, 0.5, (S, 3)) * np.asarray(L)).astype(np.float32)
+    return pos, rng.uniform(0.05, rmax, S).astype(np.float32), rng.integers(0, 5, S).astype(np.float32)
+
+
+def _closest_call(pos, r, buff):
+    p, q = pos.astype(np.float64), r.astype(np.float64)
+    i, j = np.triu_indices(len(r), 1)
+    if i.size == 0:
+        return np.inf
+    return np.abs(np.linalg.norm(p[i] - p[j], axis=1) - (q[i] + q[j] + buff)).min()
+
+
+# member counts on both sides of the tiles (256), one sphere, and a box of
+# 90,000 blocks (more than a CTA counts in shared memory)
+CROWDS = [(1, (2.0, 2.0, 2.0), 0.4), (2, (2.0, 2.0, 2.0), 0.8), (255, (2.0, 2.0, 2.0), 0.2),
+          (256, (2.0, 2.0, 2.0), 0.2), (257, (2.0, 2.0, 2.0), 0.2), (513, (2.0, 2.0, 2.0), 0.1),
+          (900, (10.0, 10.0, 900.0), 1.0)]
+
+
+def _crowd_seed(S, L, rmax):
+    return next(s for s in range(100) if _closest_call(*_crowd(S, L, s, rmax)[:2], np.float32(0.03)) > 1e-6)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("S,L,rmax", CROWDS)
+def test_device_collision_at_tile_edges(S, L, rmax):
+    pytest.importorskip("torch")
+    from nozomi_b200.collide import detect_collision
+    pos, r, fid = _crowd(S, L, _crowd_seed(S, L, rmax), rmax)
+    got = detect_collision(pos, r, fid, *L, buff=0.03)
+    np.testing.assert_array_equal(got.cpu().numpy(), collide(pos, r, fid, *L, buff=0.03))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("what,value", [("pos", np.nan), ("pos", np.inf), ("radius", np.nan), ("radius", -np.inf)])
+def test_device_collision_refuses_non_finite_spheres(what, value):
+    pytest.importorskip("torch")
+    from nozomi_b200._lib import NozomiError
+    from nozomi_b200.collide import detect_collision
+    pos, r, fid = _crowd(300, (5.0, 5.0, 5.0), 1, 0.5)
+    (pos[200] if what == "pos" else r[200:201])[0] = value
+    with pytest.raises(NozomiError, match="finite"):
+        detect_collision(pos, r, fid, 5.0, 5.0, 5.0)
