@@ -17,6 +17,7 @@
 #ifndef NOZOMI_B200_H
 #define NOZOMI_B200_H
 
+#include <stddef.h>
 #include <stdint.h>
 
 #ifdef __cplusplus
@@ -44,6 +45,9 @@ extern "C" {
  * per-entry record lists) */
 #define NZ_LIST_IDX16 64    /* substrates with idx_bytes 2 */
 #define NZ_LIST_IDX32 128   /* substrates with idx_bytes 4 */
+
+/* added to nz_substrate.idx_bytes: near_sph4 holds packed near entries (nz_cells_pack) */
+#define NZ_NEAR_PACKED 256
 
 /* per-walker flag bits */
 #define NZ_FLAG_DRAWS_EXHAUSTED 1
@@ -102,6 +106,11 @@ typedef struct nz_substrate {
      * (nz_cells_index).  Entries ascending by record are ascending by
      * structure, so a walker labelled L stops at the first record at or
      * beyond sid_start[L + 1]: no structure id is read per entry. */
+    /* idx_bytes may carry NZ_NEAR_PACKED (2 + NZ_NEAR_PACKED or 4 +
+     * NZ_NEAR_PACKED): near_sph4 then holds the packed entries of the near
+     * lists (nz_cells_pack, 16-byte aligned; near_items given), which the
+     * fused walk's near filter reads instead of the records.  They change how
+     * fast entries are passed over, never a result. */
     int idx_bytes;
     const void* cell_idx;
     const void* near_idx;
@@ -223,6 +232,24 @@ int nz_cells_gather(const float* spheres, int S, const int* items, int n_items, 
  * (int32). */
 int nz_cells_index(const int* items, int n_items, const int* perm, int S, const int* cell_start,
                    const int* cell_count, int ncell, void* idx, int idx_bytes, void* stream);
+
+/* Packed near entries of index lists: per cell its entries two by two, each
+ * pair 16 bytes of half-precision numbers (x, x', y, y', z, z', R, R'):
+ * the centres relative to the cell's centre, and the radii R of balls that,
+ * grown by 2 % of the reach, hold the (r + tol) balls with 2 nm and the
+ * rounding of a half-precision distance to spare (margin: the near lists'
+ * membership margin, which bounds the walker's distance and reach where the
+ * near lists are taken).  After the pairs, a squared safe radius per record:
+ * a walker of the record's structure whose segment stays that close to the
+ * record's centre meets no sphere.  idx, start, count: the near lists, laid
+ * out without gaps (start the exclusive scan of count); full_*: the cell
+ * lists.  pack: nz_cells_pack_bytes(n_items, ncell, S) bytes, 16-byte
+ * aligned; nz_substrate.near_items must then be n_items.  Grids with a cell
+ * edge above 1e4 um are refused. */
+size_t nz_cells_pack_bytes(int n_items, int ncell, int S);
+int nz_cells_pack(const float* rec4, const int* rec_sid, int S, const void* idx, int idx_bytes, const int* start,
+                  const int* count, int n_items, const void* full_idx, const int* full_start, const int* full_count,
+                  const nz_grid* grid, float margin, void* pack, void* stream);
 
 /* ---- a12: substrate ingestion on the device — split_matrix_to_list
  * (utils/common_utils.py:41-55) and createBoundaryZ / create_pad

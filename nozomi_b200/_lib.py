@@ -20,6 +20,7 @@ LIB_PATH = Path(__file__).resolve().parent / ("libnozomi_b200_debug.so" if DEBUG
 NZ_OK, NZ_ERR_ARG, NZ_ERR_CUDA, NZ_ERR_CAPACITY, NZ_ERR_UNSEEDED = 0, 1, 2, 3, 4
 MODE_SIG, MODE_PHASE, MODE_PHI, MODE_MOMENTS, MODE_TANGENT64 = 1, 2, 4, 8, 16
 LIST_IDX16, LIST_IDX32 = 64, 128  # nz_walk_batch: the jobs' list format (none: per-entry records)
+NEAR_PACKED = 256  # added to Substrate.idx_bytes: near_sph4 holds packed near entries (nz_cells_pack)
 FLAG_DRAWS_EXHAUSTED, FLAG_ITER_CAP, FLAG_UNSEEDED, FLAG_BOUNDS, FLAG_STAGE_TIMEOUT = 1, 2, 4, 8, 16
 MAX_STAGE_RECORDS = 12288  # nz_walk_batch_staged: records a CTA stages in shared memory at most
 FUSED_THREADS = 128       # walkers per CTA / per work item of the fused and batched walks
@@ -87,6 +88,8 @@ SIGNATURES = {
     "nz_segments_fill": (_i, [_P, _i, _d, _d, _d, _i, _i, _i, _i, _P, _P]),
     "nz_cells_gather": (_i, [_P, _i, _P, _i, _P, _P, _i, _P, _P, _P]),
     "nz_cells_index": (_i, [_P, _i, _P, _i, _P, _P, _i, _P, _i, _P]),
+    "nz_cells_pack_bytes": (ctypes.c_size_t, [_i, _i, _i]),
+    "nz_cells_pack": (_i, [_P, _P, _i, _P, _i, _P, _P, _i, _P, _P, _P, _P, _f, _P, _P]),
     "nz_collide_scratch_bytes": (ctypes.c_size_t, [_i, _P]),
     "nz_collide_cells": (_i, [_P, _P, _i, _P, _P, _P, ctypes.c_size_t, _P]),
     "nz_collide_pairs": (_i, [_P, _P, _P, _i, _P, _f, _P, _i, _P, _i, _P, _P, ctypes.c_size_t, _P]),

@@ -110,12 +110,13 @@ extern "C" int nz_walk_step(const nz_substrate* sub, const nz_walkers* wk, int m
   a.n_scatter = wk->n_scatter;
   a.flags = wk->flags;
   // index lists, where the substrate has them, hold the same members
-  if ((sub->idx_bytes == 2 || sub->idx_bytes == 4) && sub->cell_idx && sub->rec4 && sub->rec_sid && sub->sid_start &&
-      aligned16(sub->rec4) && (sub->idx_bytes == 4 || sub->S <= 65536))
+  const int width = sub->idx_bytes & ~NZ_NEAR_PACKED;
+  if ((width == 2 || width == 4) && sub->cell_idx && sub->rec4 && sub->rec_sid && sub->sid_start &&
+      aligned16(sub->rec4) && (width == 4 || sub->S <= 65536))
     return launch_plain_lists(a,
                               PlainLists{sub->cell_idx, reinterpret_cast<const float4*>(sub->rec4), sub->rec_sid,
                                          sub->sid_start},
-                              sub->idx_bytes, static_cast<cudaStream_t>(stream));
+                              width, static_cast<cudaStream_t>(stream));
   walk_plain_kernel<<<(wk->N + 255) / 256, 256, 0, static_cast<cudaStream_t>(stream)>>>(a);
   return check_launch("walk_plain_kernel");
 }
@@ -168,9 +169,13 @@ static int check_fused_sub(const nz_substrate* sub, const char* who) {
   int rc = check_substrate(sub, who);
   if (rc) return rc;
   if (sub->idx_bytes != 0) {
-    if (sub->idx_bytes != 2 && sub->idx_bytes != 4)
+    const bool packed = (sub->idx_bytes & NZ_NEAR_PACKED) != 0;
+    const int width = sub->idx_bytes & ~NZ_NEAR_PACKED;
+    if (width != 2 && width != 4)
       return set_error(NZ_ERR_ARG, "%s: idx_bytes %d is not 0, 2 or 4", who, sub->idx_bytes);
-    if (sub->idx_bytes == 2 && sub->S > 65536)
+    if (packed && (!sub->near_idx || !sub->near_sph4 || !aligned16(sub->near_sph4)))
+      return set_error(NZ_ERR_ARG, "%s: packed near entries need near lists and a 16-byte aligned near_sph4", who);
+    if (width == 2 && sub->S > 65536)
       return set_error(NZ_ERR_ARG, "%s: %d spheres do not fit 16-bit indices", who, sub->S);
     if (!sub->cell_idx || !sub->rec4 || !sub->rec_sid || !sub->sid_start)
       return set_error(NZ_ERR_ARG, "%s: index lists need cell_idx, rec4, rec_sid and sid_start", who);
@@ -195,6 +200,19 @@ static int batch_list_kind(int mode) {
   return (mode & NZ_LIST_IDX16) ? 2 : (mode & NZ_LIST_IDX32) ? 4 : 0;
 }
 
+// Walkers a warp of the single-substrate fused walk: 32, fewer for few
+// walkers.  A warp's step takes as long as its slowest lanes together, so
+// while warps are scarce, spreading the walkers over up to about two warps a
+// scheduler (1,250 on 148 SMs) shortens every step: 100 axons, 400 steps take
+// 1.92 ms for 2,003 walkers at 32 a warp, 1.73 / 1.47 / 1.30 / 1.25 / 1.36 at
+// 16 / 8 / 4 / 2 / 1; 5,000: 2.02, 1.79, 1.63, 1.57 at 4; 20,000: 2.12, 2.08
+// at 16, 2.22 at 8; 40,000: 2.52, 2.57 at 16.
+static int fused_lanes(int N) {
+  int lanes = 1;
+  while (lanes < 32 && N > lanes * 1250) lanes *= 2;
+  return lanes;
+}
+
 extern "C" int nz_walk_fused(const nz_substrate* sub, const nz_state* st, int mode, float dt, const float* G,
                              const float* Garea, int step0, int step1, const nz_draws* draws, double* moments,
                              void* stream) {
@@ -213,9 +231,10 @@ extern "C" int nz_walk_fused(const nz_substrate* sub, const nz_state* st, int mo
   if (step0 < 0 || step1 < step0) return set_error(NZ_ERR_ARG, "nz_walk_fused: bad step range");
   if (st->N == 0 || step1 == step0) return NZ_OK;
   const JobDev j = make_job(*sub, G, Garea, step1, dt, *draws, mode, *st, moments);
-  const int n_items = (st->N + kFusedThreads - 1) / kFusedThreads;
-  return launch_fused(mode, sub->idx_bytes, j, nullptr, nullptr, n_items, step0, step1, nullptr, n_items,
-                      kFusedThreads, static_cast<cudaStream_t>(stream));
+  const int lanes = fused_lanes(st->N), per = kFusedThreads / 32 * lanes;
+  const int n_items = (st->N + per - 1) / per;
+  return launch_fused(mode, sub->idx_bytes & ~NZ_NEAR_PACKED, j, nullptr, nullptr, n_items, step0, step1, nullptr,
+                      n_items, kFusedThreads, static_cast<cudaStream_t>(stream), lanes);
 }
 
 extern "C" size_t nz_walk_fused_moments_scratch_bytes(int N, int nsteps) {
@@ -243,9 +262,10 @@ extern "C" int nz_walk_fused_moments(const nz_substrate* sub, const nz_state* st
   const cudaStream_t cs = static_cast<cudaStream_t>(stream);
   JobDev j = make_job(*sub, G, Garea, step1, dt, *draws, mode, *st, nullptr);
   j.disp = scratch;
-  const int n_items = (st->N + kFusedThreads - 1) / kFusedThreads;
-  rc = launch_fused(mode | kModeDisp, sub->idx_bytes, j, nullptr, nullptr, n_items, step0, step1, nullptr, n_items,
-                    kFusedThreads, cs);
+  const int lanes = fused_lanes(st->N), per = kFusedThreads / 32 * lanes;
+  const int n_items = (st->N + per - 1) / per;
+  rc = launch_fused(mode | kModeDisp, sub->idx_bytes & ~NZ_NEAR_PACKED, j, nullptr, nullptr, n_items, step0, step1,
+                    nullptr, n_items, kFusedThreads, cs, lanes);
   if (rc) return rc;
   const int gx = min(64, (st->N + 255) / 256);
   disp_moments_kernel<<<dim3(gx, step1 - step0), 256, 0, cs>>>(scratch, st->N, moments + size_t(step0) * 6);

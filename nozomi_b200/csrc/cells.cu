@@ -8,7 +8,9 @@
 // boundary distances of its bounding box are below jump_tol.  The predicate is
 // separable per axis and, per axis, monotone in the cell index, so each sphere
 // enumerates only the box of cells it can belong to.
+#include <cmath>
 #include <cstdint>
+#include <cuda_fp16.h>
 #include "kernels.cuh"
 
 namespace nz {
@@ -685,6 +687,115 @@ __global__ void index_fill_kernel(const int* __restrict__ items, int n, const in
   idx[k] = T(perm ? perm[s] : s);
 }
 
+// Packed near entries (nz_cells_pack): the near filter of the fused walk in
+// half precision, two spheres an instruction (near_bits_packed in
+// walk_fused.cu).  An entry stores its sphere's centre relative to the cell's
+// centre and the radius R of the ball the filter tests,
+//   R = r (1 + 5e-5) + tol + 2 nm + E,  rounded up,
+// with E a bound on the error of the filter's distance.  With u = 2^-11 (one
+// rounding), rho = r + tol, M the near margin (distance of the walker from
+// the cell plus reach <= M wherever the near lists are taken), h half the
+// cell's diagonal and m = h + 2 M + rho >= the lengths of the walker's and
+// the sphere's positions and of their difference d, for a sphere whose true
+// distance from the segment is within its ball:
+//   rounding of the two positions and of d              3 u m
+//   of the segment's direction and length               2 u M
+//   of d^2, d.e, s (s + 2 d.e) and their sum, at |d| <= rho + M,
+//   as a distance                              u (2 rho + 7 M + 5.5 M^2 / rho)
+//   of R + 2 % reach and its square                     2 u rho
+// E is their sum and 15 % more (10 nm for r = 1 um, 0.5 um cells and margin).
+// Spheres that half precision holds badly (R above 100 um, centres beyond
+// 200 um) get R = inf: always near.
+__device__ __forceinline__ void pack_entry(float4 c, double ox, double oy, double oz, double h, double M, __half* v) {
+  const double x = double(c.x) - ox, y = double(c.y) - oy, z = double(c.z) - oz;
+  const double u = 1.0 / 2048, rho = double(c.w) + double(kTol), m = h + 2 * M + rho;
+  const double E = 1.15 * u * (3 * m + 9 * M + 4 * rho + 5.5 * M * M / rho);
+  const double R = double(c.w) * (1.0 + 5e-5) + double(kTol) + 2e-3 + E;
+  const bool fits = R <= 100.0 && fabs(x) <= 200.0 && fabs(y) <= 200.0 && fabs(z) <= 200.0;
+  v[0] = __float2half_rn(fits ? float(x) : 0.0f);
+  v[1] = __float2half_rn(fits ? float(y) : 0.0f);
+  v[2] = __float2half_rn(fits ? float(z) : 0.0f);
+  v[3] = fits ? __float2half_ru(__double2float_ru(R)) : __ushort_as_half(0x7c00);
+}
+
+template <typename T>
+__global__ void cells_pack_kernel(const float4* __restrict__ rec4, const T* __restrict__ idx,
+                            const int* __restrict__ start, const int* __restrict__ count, Grid g, double h, double M,
+                            uint4* __restrict__ pack) {
+  const int nx = int(g.nLx), ny = int(g.nLy), ncell = nx * ny * int(g.nLz);
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= ncell) return;
+  const int n = count[c], s = start[c];
+  // the cell's centre as the walk forms it (step_cell's low corner plus half an edge)
+  const double ox = double(float(c % nx) * g.dLx - g.Lx / 2) + 0.5 * g.dLx;
+  const double oy = double(float((c / nx) % ny) * g.dLy - g.Ly / 2) + 0.5 * g.dLy;
+  const double oz = double(float(c / (nx * ny)) * g.dLz - g.Lz / 2) + 0.5 * g.dLz;
+  uint4* out = pack + ((s + c + 1) >> 1);
+  for (int i = 0; i < n; i += 2) {
+    __half a[4], b[4];
+    pack_entry(__ldg(rec4 + int(idx[s + i])), ox, oy, oz, h, M, a);
+    if (i + 1 < n) {
+      pack_entry(__ldg(rec4 + int(idx[s + i + 1])), ox, oy, oz, h, M, b);
+    } else {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) b[k] = a[k];
+    }
+    uint32_t w[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) w[k] = uint32_t(__half_as_ushort(a[k])) | (uint32_t(__half_as_ushort(b[k])) << 16);
+    out[i >> 1] = make_uint4(w[0], w[1], w[2], w[3]);
+  }
+}
+
+// Safe balls of the records (nz_cells_pack): a ball around a sphere's centre
+// such that a walker of the sphere's structure whose segment stays in it
+// takes its whole jump.  It lies 2 nm + 0.005 % of r inside the sphere (the
+// fraction of the sphere itself is then at least the jump, by far more than
+// the rounding of the reference's arithmetic) and as far, and 1 % of r more,
+// outside the (r + tol) ball of every sphere of a lower structure that such
+// a walker's list can hold (none of them contains it or stops it).  The walk
+// uses them in iterations that stay within the near margin of the walker's
+// cell, so a point where a lower sphere meets this one lies within that
+// margin of the box, and both spheres are in the full list (membership
+// margin larger than the near one) of the cell the point falls or is clamped
+// to: the lists of the cells that the sphere's box covers hold them all.  A
+// warp per record; the squared radius is stored, -1 for none.
+template <typename T>
+__global__ void cells_safe_kernel(const float4* __restrict__ rec4, const int* __restrict__ rec_sid, int S,
+                                  const T* __restrict__ idx, const int* __restrict__ start,
+                                  const int* __restrict__ count, Grid g, float* __restrict__ safe) {
+  const int k = int((blockIdx.x * size_t(blockDim.x) + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+  if (k >= S) return;
+  const float4 c = __ldg(rec4 + k);
+  const int sid = __ldg(rec_sid + k);
+  float best = c.w * 0.99995f - 2e-3f;
+  const float reach = c.w + 0.01f;
+  const int nx = int(g.nLx), ny = int(g.nLy);
+  const int x0 = int(fminf(g.nLx - 1, fmaxf(0.f, floorf((c.x - reach + g.Lx / 2) / g.dLx))));
+  const int x1 = int(fminf(g.nLx - 1, fmaxf(0.f, floorf((c.x + reach + g.Lx / 2) / g.dLx))));
+  const int y0 = int(fminf(g.nLy - 1, fmaxf(0.f, floorf((c.y - reach + g.Ly / 2) / g.dLy))));
+  const int y1 = int(fminf(g.nLy - 1, fmaxf(0.f, floorf((c.y + reach + g.Ly / 2) / g.dLy))));
+  const int z0 = int(fminf(g.nLz - 1, fmaxf(0.f, floorf((c.z - reach + g.Lz / 2) / g.dLz))));
+  const int z1 = int(fminf(g.nLz - 1, fmaxf(0.f, floorf((c.z + reach + g.Lz / 2) / g.dLz))));
+  for (int p = z0; p <= z1; ++p)
+    for (int m = y0; m <= y1; ++m)
+      for (int n = x0; n <= x1; ++n) {
+        const int cell = (p * ny + m) * nx + n;
+        const int s = start[cell], e = s + count[cell];
+        for (int i = s + lane; i < e; i += 32) {
+          const int o = int(idx[i]);
+          if (o >= S || __ldg(rec_sid + o) >= sid) continue;
+          const float4 d = __ldg(rec4 + o);
+          const float ex = d.x - c.x, ey = d.y - c.y, ez = d.z - c.z;
+          const float gap = sqrtf(ex * ex + ey * ey + ez * ez) * 0.99999f - d.w * 1.00005f;
+          best = fminf(best, gap - 2e-3f - kTol - 0.01f * c.w);
+        }
+      }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) best = fminf(best, __shfl_xor_sync(0xffffffffu, best, o));
+  if (lane == 0) safe[k] = best > 0.0f ? best * best : -1.0f;
+}
+
 // Exclusive scan of in[lo, hi) into out[lo, hi) by one CTA (1024 threads, 8
 // items per thread per pass), starting from carry; returns the range's total
 // (in every thread).
@@ -981,4 +1092,50 @@ extern "C" int nz_cells_index(const int* items, int n_items, const int* perm, in
     if (rc) return rc;
     return sort_lists(cell_start, cell_count, ncell, S, p, st);
   }
+}
+
+extern "C" size_t nz_cells_pack_bytes(int n_items, int ncell, int S) {
+  if (n_items < 0 || ncell < 0 || S < 0) return 0;
+  return pack_pairs(n_items, ncell) * 16 + size_t(S) * sizeof(float);
+}
+
+extern "C" int nz_cells_pack(const float* rec4, const int* rec_sid, int S, const void* idx, int idx_bytes,
+                             const int* start, const int* count, int n_items, const void* full_idx,
+                             const int* full_start, const int* full_count, const nz_grid* grid, float margin,
+                             void* pack, void* stream) {
+  int rc = check_grid(grid, "nz_cells_pack");
+  if (rc) return rc;
+  if (S < 0 || n_items < 0 || (idx_bytes != 2 && idx_bytes != 4) || !(margin > 0.0f) || !pack ||
+      (reinterpret_cast<uintptr_t>(pack) & 15) || !start || !count || !full_start || !full_count ||
+      (S > 0 && (!rec4 || !rec_sid || !full_idx)) || (n_items > 0 && !idx) ||
+      (reinterpret_cast<uintptr_t>(rec4) & 15))
+    return set_error(NZ_ERR_ARG, "nz_cells_pack: bad arguments (S=%d items=%d idx_bytes=%d)", S, n_items, idx_bytes);
+  if (!(grid->dLx <= 1e4f && grid->dLy <= 1e4f && grid->dLz <= 1e4f))
+    return set_error(NZ_ERR_ARG, "nz_cells_pack: cell edges above 1e4 um");
+  const long long ncell = 1ll * grid->nx * grid->ny * grid->nz;
+  if (ncell + n_items > 0x7fffffffll) return set_error(NZ_ERR_ARG, "nz_cells_pack: too many cells and entries");
+  const Grid g{grid->Lx, grid->Ly, grid->Lz, grid->dLx, grid->dLy, grid->dLz, float(grid->nx), float(grid->ny),
+               float(grid->nz)};
+  const double h = 0.5 * sqrt(double(g.dLx) * g.dLx + double(g.dLy) * g.dLy + double(g.dLz) * g.dLz);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const unsigned blocks = unsigned((ncell + 127) / 128);
+  const float4* r = reinterpret_cast<const float4*>(rec4);
+  uint4* out = static_cast<uint4*>(pack);
+  float* safe = reinterpret_cast<float*>(out + pack_pairs(n_items, int(ncell)));
+  const unsigned sblocks = unsigned((size_t(S) * 32 + 255) / 256);
+  if (idx_bytes == 2)
+    cells_pack_kernel<<<blocks, 128, 0, st>>>(r, static_cast<const uint16_t*>(idx), start, count, g, h,
+                                              double(margin), out);
+  else
+    cells_pack_kernel<<<blocks, 128, 0, st>>>(r, static_cast<const int*>(idx), start, count, g, h, double(margin),
+                                              out);
+  rc = check_launch("cells_pack_kernel");
+  if (rc || S == 0) return rc;
+  if (idx_bytes == 2)
+    cells_safe_kernel<<<sblocks, 256, 0, st>>>(r, rec_sid, S, static_cast<const uint16_t*>(full_idx), full_start,
+                                               full_count, g, safe);
+  else
+    cells_safe_kernel<<<sblocks, 256, 0, st>>>(r, rec_sid, S, static_cast<const int*>(full_idx), full_start,
+                                               full_count, g, safe);
+  return check_launch("cells_safe_kernel");
 }

@@ -65,13 +65,10 @@ constexpr size_t kSmemPerSm = 228 * 1024;  // shared memory an SM can give its C
 #define NZ_FUSED_MIN_BLOCKS 3
 #endif
 constexpr int kFusedMinBlocks = NZ_FUSED_MIN_BLOCKS;  // 256-thread CTAs per SM the register budget is sized for
-#ifndef NZ_SCAN_UNROLL
-#define NZ_SCAN_UNROLL 4
-#endif
-// list entries loaded together in the scan's first pass: 4 measured fastest
-// on both the batched and the packed workloads (1, 2, 4, 8 tried)
-constexpr int kScanUnroll = NZ_SCAN_UNROLL;
-static_assert(32 % kScanUnroll == 0, "the scan unroll must divide 32");
+// Pairs of the packed near entries of n_items entries in ncell cells: the
+// pairs of cell c begin at (start[c] + c + 1) / 2; the walk may read a pair
+// past a cell's last one.
+__host__ __device__ inline size_t pack_pairs(int n_items, int ncell) { return (size_t(n_items) + size_t(ncell)) / 2 + 4; }
 constexpr int kMomentSteps = 256;  // steps per launch in NZ_MODE_MOMENTS (shared-memory staging)
 // Internal mode bit (nz_walk_fused_moments only): at each step end the fused
 // walk stores the walker's float displacement from its origin; a reduction
@@ -112,6 +109,8 @@ struct JobDev {
   // index form of the lists (nz_substrate.idx_bytes > 0)
   const void* idx;
   const void* near_idx;
+  const uint4* near_pack;  // packed near entries (NZ_NEAR_PACKED), or null
+  const float* rec_safe;   // with them: squared safe radius of each record
   const float4* rec4;
   const int* rec_sid;
   const int* sid_start;
@@ -122,7 +121,8 @@ struct JobDev {
 
 __host__ __device__ JobDev make_job(const nz_substrate& sub, const float* G, const float* Garea, int nsteps, float dt,
                                     const nz_draws& d, int mode, const nz_state& st, double* moments);
-// lk: list kind, 0 (per-entry records), 2 or 4 (index lists of that width)
+// lk: list kind, 0 (per-entry records), 2 or 4 (index lists of that width).
+// stage_cap: batched walk, records a CTA stages; single job, walkers a warp.
 int launch_fused(int mode, int lk, const JobDev& single, const nz_job* jobs, const nz_item* items, int n_items,
                  int step0, int step1, int* queue, int grid, int threads, cudaStream_t st, int stage_cap = 0);
 int occupancy_fused(int mode, int lk, int threads, int* blocks_per_sm, int stage_cap = 0);

@@ -13,22 +13,24 @@
 //    pass proves that label (some containing sphere of that structure, none of
 //    a lower one) or the iteration is redone with the recomputed label, so the
 //    result is the reference's;
-//  * the list is scanned in two passes.  The first, predicated and over
-//    every entry, marks the near spheres: a sphere whose (r + tol) ball lies
-//    more than 2 % + 2 nm beyond this iteration's reach |j| * jump_remaining
-//    neither contains the walker nor can lower the jump fraction (its root
-//    exceeds jump_remaining), so it is dropped.  The second, over the near
-//    spheres of a 32-entry chunk only, runs the reference's inside test and
-//    the fractions, so a warp pays for the most near spheres of any lane
-//    rather than for every entry twice;
+//  * a walker whose segment stays in the safe ball of the sphere that held it
+//    last (nz_cells_safe) takes its whole jump and scans nothing: three of
+//    four iterations of walkers inside axons;
+//  * the others scan their list in two passes.  The first marks the near
+//    spheres, those whose (r + tol) ball comes within 2 nm and 2 % of the
+//    reach of the segment ahead, from packed entries in half precision, two
+//    spheres an instruction; any other sphere neither contains the walker nor
+//    can lower the jump fraction.  The second runs the reference's inside
+//    test and the fractions for the marked ones only;
 //  * the near lists (the same cell grid with a smaller margin) serve every
-//    iteration whose reach fits their margin; the full lists the rest;
-//  * the cell list entries carry their sphere's (cx, cy, cz, r) and structure
-//    id inline (one 16-byte and one 4-byte read-only load per entry; walkers
-//    in the box read no structure id);
+//    iteration whose reach fits their margin; the full lists the rest, scanned
+//    by the whole warp together;
+//  * list entries are record indices (or, in record lists, carry their
+//    sphere's record and structure id inline); lists without packed entries
+//    are walked a lane a walker (walk_one);
 //  * each iteration has one draw site (the scatter draw of this step or the
 //    first draw of the next), and the inside and outside fractions share one
-//    instruction stream (step_either);
+//    instruction stream with one division (step_one);
 //  * phase is accrued as the 3-vector Phi = sum_n G_n p_n with Kahan
 //    compensation, the wrap correction on the wrapped axis only; every
 //    direction's phase is u_d . Phi (the reference's per-direction sums
@@ -37,6 +39,7 @@
 //    trajectory does not depend on which thread, CTA or launch runs it.
 #include <algorithm>
 #include <cstdint>
+#include <cuda_fp16.h>
 #include <mutex>
 #include "kernels.cuh"
 
@@ -47,44 +50,203 @@ struct ScanOut {
   bool any_in;
 };
 
-// One list entry: its sphere's record and a key.  Record lists (LK 0): the
-// record inline, the key the structure id (-1 for a walker in the box, which
-// reads none).  Index lists (LK 2 or 4): the key the record index, the record
-// read from the substrate's record array.  In the bounds-checked build a
-// record index outside [0, S) sets oob and reads nothing: the entry becomes
-// a NaN record that is neither near nor containing, with a key that stops
-// nothing.
-// The records of a job staged in shared memory (staged batched walk only).
+// Dynamic shared memory: the records of a job (staged batched walk only),
+// then, in the phase modes, each thread's walker's Phi with its compensation
+// (a float4 per thread: Phi, compensation x; then a float2 per thread:
+// compensation y, z), or, in the moment modes, its origin (a float4 per
+// thread).  They are touched once a step and would hold registers through the
+// collision pass.
 extern __shared__ __align__(16) float4 s_stage[];
+template <int MODE>
+constexpr size_t phi_bytes(int threads) {
+  return (MODE & NZ_MODE_PHI) ? size_t(threads) * 24 : (MODE & (NZ_MODE_MOMENTS | kModeDisp)) ? size_t(threads) * 16 : 0;
+}
 
+// Record `key` of the substrate's record array (SH: the staged copy).  In
+// the bounds-checked build an index outside [0, S) sets oob and reads
+// nothing: the entry becomes a NaN record that is neither near nor
+// containing, with a key that stops nothing.
+template <bool SH>
+__device__ __forceinline__ float4 record(const float4* __restrict__ rec, int S, int& key, int& oob) {
+  if (kCheckBounds && (key < 0 || key >= S)) {
+    oob = 1;
+    key = -1;
+    return make_float4(__int_as_float(0x7fc00000), 0.f, 0.f, 0.f);
+  }
+  if constexpr (SH) return s_stage[key];  // SH: the job's records were copied there
+  return __ldg(rec + key);
+}
+
+// One list entry: its sphere's record and a key.  Record lists (LK 0): the
+// record inline, the key the structure id.  Index lists (LK 2 or 4): the key
+// the record index, the record read from the substrate's record array.  The
+// entries of a cell ascend by key.  In either form the entries of structure
+// L have keys in [lo, hi) (label_bounds): key < hi is "structure <= L" and
+// key < lo "structure < L"; for a walker in the box every key is below lo.
 template <int LK, bool SH>
 __device__ __forceinline__ void entry(const void* __restrict__ list, const float4* __restrict__ rec,
-                                      const int* __restrict__ sid, int k, bool box, int S, int& oob, int& key,
-                                      float4& c) {
+                                      const int* __restrict__ sid, int k, int S, int& oob, int& key, float4& c) {
   if constexpr (LK == 0) {
-    key = box ? -1 : __ldg(sid + k);
+    key = __ldg(sid + k);
     c = __ldg(rec + k);
   } else {
     if constexpr (LK == 2) key = int(__ldg(static_cast<const unsigned short*>(list) + k));
     else key = __ldg(static_cast<const int*>(list) + k);
-    if (kCheckBounds && (key < 0 || key >= S)) {
-      oob = 1;
-      key = -1;
-      c = make_float4(__int_as_float(0x7fc00000), 0.f, 0.f, 0.f);
-      return;
-    }
-    if constexpr (SH) c = s_stage[key];  // SH: the job's records were copied into s_stage
-    else c = __ldg(rec + key);
+    c = record<SH>(rec, S, key, oob);
   }
 }
 
-// One pass over a cell's list under assumed label L.  Returns false when the
-// walker's label is not L (then nothing in `o` is used).  The entries of a
-// cell are ordered by structure id: the pass ends at the first entry of a
-// structure above L (the reference skips those spheres, :805-806).  In index
-// form an entry's structure is compared through its record index: records
-// [lo, hi) are structure L's, so key < hi is "structure <= L" and key < lo
-// "structure < L".
+// The reference's collision pass over one cell's list for one walker of
+// known label (sim3d_kernel.cu:800-830), lane by lane: only for the rare
+// iteration whose label had to be corrected.
+template <int LK, bool T64, bool SH>
+__device__ __noinline__ void scan_lane(const void* __restrict__ list, const float4* __restrict__ rec,
+                                          const int* __restrict__ sid, int start, int count, int lo, int hi, float x,
+                                          float y, float z, float a, float jx, float jy, float jz, int S, int& oob,
+                                          ScanOut& o) {
+  o.fin = 0.0f;
+  o.fout = kBig;
+  o.any_in = false;
+  for (int i = 0; i < count; ++i) {
+    int key;
+    float4 c;
+    entry<LK, SH>(list, rec, sid, start + i, S, oob, key, c);
+    if (key >= hi) break;
+    const float dx = x - c.x, dy = y - c.y, dz = z - c.z;
+    const bool inside = dx * dx + dy * dy + dz * dz - c.w * c.w < 0;
+    if (inside || key < lo) {
+      const float f = step_either_t<T64>(inside, dx, dy, dz, c.w, a, jx, jy, jz);
+      if (inside) {
+        o.any_in = true;
+        if (o.fin < f) o.fin = f;
+      } else if (f < o.fout) {
+        o.fout = f;
+      }
+    }
+  }
+}
+
+// The near filter's view of one walker's iteration.
+struct Reach {
+  float mx, my, mz, m2;  // twice the displacement left in this step; the displacement's squared length
+  float k;               // -1/2 over that square
+  float slack;
+};
+
+// Whether a sphere's (r + tol) ball, grown by 2 nm, 0.005 % of r and 2 % of
+// the reach (or by `slack`), meets the segment that the walker would walk in
+// this iteration.  A sphere farther from the whole segment neither contains
+// the walker nor can stop it: its root lies beyond the segment's end, or the
+// ray misses it, by far more than the rounding of the reference's
+// arithmetic.  A filter, not the reference's arithmetic: fused multiply-adds
+// are fine here.
+__device__ __forceinline__ bool is_near(const Reach& g, float x, float y, float z, float4 c) {
+  const float dx = x - c.x, dy = y - c.y, dz = z - c.z;
+  const float d2 = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, dz * dz));
+  const float dm = __fmaf_rn(dx, g.mx, __fmaf_rn(dy, g.my, dz * g.mz));
+  const float t = __saturatef(dm * g.k);  // the segment's nearest point to the centre
+  const float ro = __fmaf_rn(c.w, 1.00005f, g.slack);
+  return __fmaf_rn(t, __fmaf_rn(t, g.m2, dm), d2) <= ro * ro;
+}
+
+// Near masks cover 32 list entries: entry i at bit (i >> 1) | (i & 1) << 4.
+__device__ __forceinline__ int bit_entry(int bit) { return 2 * (bit & 15) + (bit >> 4); }
+
+// Near mask of `n` (at most 32) entries from list position `first` on, from
+// their records; entries of a structure above the walker's are left out (keys
+// ascend).
+template <int LK, bool SH>
+__device__ __forceinline__ uint32_t near_bits(const void* __restrict__ list, const float4* __restrict__ rec,
+                                              const int* __restrict__ sid, int first, int n, int hi, int S, int& oob,
+                                              const Reach& g, float x, float y, float z) {
+  uint32_t bits = 0u;
+  bool stop = false;
+  // four entries at a time, their loads (two dependent ones each) in flight
+  // together
+  for (int i0 = 0; i0 < n && !stop; i0 += 4) {
+    int key[4];
+    float4 c[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) entry<LK, SH>(list, rec, sid, first + min(i0 + u, n - 1), S, oob, key[u], c[u]);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const bool valid = key[u] < hi && i0 + u < n;
+      stop |= key[u] >= hi;
+      bits |= valid && is_near(g, x, y, z, c[u]) ? 1u << ((i0 >> 1) + (u >> 1) + 16 * (u & 1)) : 0u;
+    }
+  }
+  return bits;
+}
+
+// The same for the packed near entries (nz_cells_pack) of up to 16 pairs, two
+// entries an instruction in half precision: px.. the position relative to
+// the cell's centre, ex.. the segment's direction, len its length, grow 2 %
+// of it.  The entries' radii hold the rounding of these distances.
+// Structures are not told apart here; entries past n are cut by the caller.
+__device__ __forceinline__ uint32_t near_bits_packed(const uint4* __restrict__ pk, int pairs, __half2 px, __half2 py,
+                                                     __half2 pz, __half2 ex, __half2 ey, __half2 ez, __half2 len,
+                                                     __half2 grow) {
+  uint32_t bits = 0u;
+  const __half2 zero = __float2half2_rn(0.0f), two = __float2half2_rn(2.0f);
+  auto test = [&](uint4 v) {
+    const __half2 dx = __hsub2(px, *reinterpret_cast<const __half2*>(&v.x));
+    const __half2 dy = __hsub2(py, *reinterpret_cast<const __half2*>(&v.y));
+    const __half2 dz = __hsub2(pz, *reinterpret_cast<const __half2*>(&v.z));
+    const __half2 d2 = __hfma2(dx, dx, __hfma2(dy, dy, __hmul2(dz, dz)));
+    const __half2 de = __hfma2(dx, ex, __hfma2(dy, ey, __hmul2(dz, ez)));
+    const __half2 t = __hmin2(__hmax2(__hneg2(de), zero), len);  // the segment's nearest point to the centre
+    const __half2 near2 = __hfma2(t, __hfma2(de, two, t), d2);
+    const __half2 ro = __hadd2(*reinterpret_cast<const __half2*>(&v.w), grow);
+    return __hle2_mask(near2, __hmul2(ro, ro));
+  };
+  for (int i = 0; i < pairs; i += 2) {  // may read one pair past the list: nz_cells_pack_bytes leaves room
+    const uint4 a = __ldg(pk + i), b = __ldg(pk + i + 1);
+    bits |= test(a) & (0x00010001u << i);
+    bits |= test(b) & (0x00020002u << i);
+  }
+  return bits;
+}
+
+// Fractions of the marked entries of one walker (bits, as near_bits marks
+// them, of the entries from list position `first` on): the reference's inside
+// test, then the fraction of a containing sphere or of a lower structure's
+// sphere.  within: the containing sphere with the largest fraction.  lower:
+// a sphere of a lower structure contains the walker.
+template <int LK, bool T64, bool SH>
+__device__ __forceinline__ void fractions(uint32_t bits, const void* __restrict__ list,
+                                          const float4* __restrict__ rec, const int* __restrict__ sid, int first,
+                                          int lo, int hi, float x, float y, float z, float a, float jx, float jy,
+                                          float jz, int S, int& oob, ScanOut& o, bool& lower, int& within) {
+  while (bits) {
+    const int i = bit_entry(__ffs(bits) - 1);
+    bits &= bits - 1u;
+    int key;
+    float4 c;
+    entry<LK, SH>(list, rec, sid, first + i, S, oob, key, c);
+    if (key >= hi) continue;
+    const bool below = key < lo;
+    const float dx = x - c.x, dy = y - c.y, dz = z - c.z;
+    const float d2 = dx * dx + dy * dy + dz * dz;
+    const bool inside = d2 - c.w * c.w < 0;
+    if (inside || below) {
+      lower |= inside && below;
+      const float f = T64 ? step_either_t<T64>(inside, dx, dy, dz, c.w, a, jx, jy, jz)
+                          : step_one(inside, dx, dy, dz, d2, c.w, a, jx, jy, jz);
+      if (inside) {
+        if (LK != 0 && (!o.any_in || o.fin < f)) within = key;
+        o.any_in = true;
+        if (o.fin < f) o.fin = f;
+      } else if (f < o.fout) {
+        o.fout = f;
+      }
+    }
+  }
+}
+
+// Lists without packed entries, each lane by itself: one pass over a cell's
+// list under assumed label L.  Returns false when the
+// walker's label is not L (then nothing in `o` is used).  Ends at the first
+// entry of a structure above L (the reference skips those spheres, :805-806).
 template <int LK, bool T64, bool SH>
 __device__ __forceinline__ bool scan_cell(const void* __restrict__ list, const float4* __restrict__ rec,
                                           const int* __restrict__ sid, int start, int count, int nstructures,
@@ -94,36 +256,34 @@ __device__ __forceinline__ bool scan_cell(const void* __restrict__ list, const f
   o.fout = kBig;
   o.any_in = false;
   bool found = false, lower = false, stop = false;
-  // A walker in the box (label nstructures) has every entry below its label:
-  // nothing to stop at and no structure to compare.
-  const bool box = L >= nstructures;
   const float slack = kTol + reach * 1.02f + 2e-3f;
+  constexpr int kUnroll = 4;
   for (int base = 0; base < count && !stop; base += 32) {
     const int m = min(32, count - base);
     // first pass: which entries are near, i.e. within (r + slack), a slack of
     // at least 2.1 nm that dwarfs the rounding of d2 and r*r, so that a far
     // sphere neither contains the walker nor lies within this iteration's
     // reach; predicated, one entry per load
-    // kScanUnroll entries are loaded together, so that their loads (two
+    // kUnroll entries are loaded together, so that their loads (two
     // dependent ones each in index form) are in flight at once; entries past
     // the first of a higher structure are invalid too (keys ascend), so a
     // batch never marks one near
     uint32_t near_mask = 0u;
-    for (int i0 = 0; i0 < m && !stop; i0 += kScanUnroll) {
-      int key[kScanUnroll];
-      float4 c[kScanUnroll];
+    for (int i0 = 0; i0 < m && !stop; i0 += kUnroll) {
+      int key[kUnroll];
+      float4 c[kUnroll];
 #pragma unroll
-      for (int u = 0; u < kScanUnroll; ++u) {
-        if (kScanUnroll == 1 || i0 + u < m) {
-          entry<LK, SH>(list, rec, sid, start + base + i0 + u, box, S, oob, key[u], c[u]);
+      for (int u = 0; u < kUnroll; ++u) {
+        if (i0 + u < m) {
+          entry<LK, SH>(list, rec, sid, start + base + i0 + u, S, oob, key[u], c[u]);
         } else {  // past the chunk: a NaN record, never near, stops nothing
           key[u] = -1;
           c[u] = make_float4(__int_as_float(0x7fc00000), 0.f, 0.f, 0.f);
         }
       }
 #pragma unroll
-      for (int u = 0; u < kScanUnroll; ++u) {
-        const bool valid = LK == 0 ? key[u] <= L : (box || key[u] < hi);
+      for (int u = 0; u < kUnroll; ++u) {
+        const bool valid = key[u] < hi;
         stop |= !valid;
         const float dx = x - c[u].x, dy = y - c[u].y, dz = z - c[u].z;
         // a filter, not the reference's arithmetic: fused multiply-adds are
@@ -140,8 +300,8 @@ __device__ __forceinline__ bool scan_cell(const void* __restrict__ list, const f
       near_mask &= near_mask - 1;
       int key;
       float4 c;
-      entry<LK, SH>(list, rec, sid, start + base + i, box, S, oob, key, c);
-      const bool below = LK == 0 ? key < L : (box || key < lo);
+      entry<LK, SH>(list, rec, sid, start + base + i, S, oob, key, c);
+      const bool below = key < lo;
       const float dx = x - c.x, dy = y - c.y, dz = z - c.z;
       const float d2 = dx * dx + dy * dy + dz * dz;
       const bool inside = d2 - c.w * c.w < 0;
@@ -165,7 +325,7 @@ __device__ __forceinline__ bool scan_cell(const void* __restrict__ list, const f
 // among the spheres containing the walker, nstructures if none.  In index
 // form the entries ascend by structure, so the first containing one decides.
 template <int LK, bool SH>
-__device__ __forceinline__ int label_of(const void* __restrict__ list, const float4* __restrict__ rec,
+__device__ __noinline__ int label_of(const void* __restrict__ list, const float4* __restrict__ rec,
                                         const int* __restrict__ sid, const int* __restrict__ rec_sid, int start,
                                         int count, int nstructures, float x, float y, float z, int S, int& oob) {
   int L = nstructures;
@@ -179,16 +339,21 @@ __device__ __forceinline__ int label_of(const void* __restrict__ list, const flo
     } else {
       int key;
       float4 c;
-      entry<LK, SH>(list, rec, sid, start + i, false, S, oob, key, c);
+      entry<LK, SH>(list, rec, sid, start + i, S, oob, key, c);
       if (inside_test(x - c.x, y - c.y, z - c.z, c.w) < 0) return __ldg(rec_sid + key);
     }
   }
   return L;
 }
 
-// Records [lo, hi) of structure L in index form (hi = lo = S for the box).
+// Keys [lo, hi) of structure L: its records in index form (lo = hi = S for
+// the box), its id in record form.
+template <int LK>
 __device__ __forceinline__ void label_bounds(const JobDev& J, int L, int& lo, int& hi) {
-  if (L >= J.nstructures) {
+  if constexpr (LK == 0) {
+    lo = L;
+    hi = L + 1;
+  } else if (L >= J.nstructures) {
     lo = hi = J.S;
   } else {
     lo = __ldg(J.sid_start + L);
@@ -196,22 +361,22 @@ __device__ __forceinline__ void label_bounds(const JobDev& J, int L, int& lo, in
   }
 }
 
-// Cell of the walker at the start of a step and the cell's low corner: the
-// clamped floor of (x + L/2) times the reciprocal cell edge.  For a walker
+// Cell of the walker at the start of a step and the cell's centre: the
+// clamped floor of x times the reciprocal cell edge plus half the cells.  For a walker
 // within a rounding error of a cell face this can be the neighbour of the
 // reference's division-based cell (cell_of); the walk's result is the same
 // with either: the near test measures the walker's distance to the cell taken
 // here, and the full lists reach jump_tol beyond their cell, so both lists
 // hold every sphere the iteration can touch or be inside.
-__device__ __forceinline__ int step_cell(const JobDev& J, float x, float y, float z, float& lox, float& loy,
-                                         float& loz) {
+__device__ __forceinline__ int step_cell(const JobDev& J, float x, float y, float z, float& mx, float& my,
+                                         float& mz) {
   const Grid& g = J.g;
-  const float cz = ref_min(g.nLz - 1, ref_max(0, floorf((z + g.Lz / 2) * J.idLz)));
-  const float cy = ref_min(g.nLy - 1, ref_max(0, floorf((y + g.Ly / 2) * J.idLy)));
-  const float cx = ref_min(g.nLx - 1, ref_max(0, floorf((x + g.Lx / 2) * J.idLx)));
-  lox = cx * g.dLx - g.Lx / 2;
-  loy = cy * g.dLy - g.Ly / 2;
-  loz = cz * g.dLz - g.Lz / 2;
+  const float cz = fminf(g.nLz - 1, fmaxf(0.f, floorf(__fmaf_rn(z, J.idLz, 0.5f * g.nLz))));
+  const float cy = fminf(g.nLy - 1, fmaxf(0.f, floorf(__fmaf_rn(y, J.idLy, 0.5f * g.nLy))));
+  const float cx = fminf(g.nLx - 1, fmaxf(0.f, floorf(__fmaf_rn(x, J.idLx, 0.5f * g.nLx))));
+  mx = __fmaf_rn(cx, g.dLx, 0.5f * (g.dLx - g.Lx));
+  my = __fmaf_rn(cy, g.dLy, 0.5f * (g.dLy - g.Ly));
+  mz = __fmaf_rn(cz, g.dLz, 0.5f * (g.dLz - g.Lz));
   return int(cz * g.nLx * g.nLy + cy * g.nLx + cx);
 }
 
@@ -251,7 +416,340 @@ __device__ __forceinline__ void jump_of(const JobDev& J, uint32_t wid, int s, in
   jz = ds * n2;
 }
 
-// Steps [s0, s1) of walker w.  Registers hold position, label, Phi and its
+// Steps [s0, s1) of the walkers of one warp, walker w in each live lane; all
+// 32 lanes run the loop together until the last one is done (they share the
+// scan of full lists).  Bound by issue slots and the latency of the list
+// loads, with 80 registers a thread (6 warps a scheduler; 96 registers
+// without the last spills are slower, 64 with more of them too): 8e8
+// walker-steps on a packed substrate took 49.5 ms with every entry's record
+// filtered in single precision against the reach, and up to five fractions
+// for a warp's worst lane; 40.4 ms so.  Tried: all lanes' entries, or their
+// marked ones, pooled over the warp in shared memory (56.3, 48.5 ms).  Registers hold position, label, Phi and
+// its compensation and the step's jump; the origin (spins0) and the flag word
+// stay in memory and are updated in place on the rare wrap / iteration-cap
+// events (except with moments, which read the origin every step).
+template <int MODE, int LK, bool SH>
+__device__ __forceinline__ void walk_warp(const JobDev& J, bool live, int w, int s0, int s1,
+                                          double* s_mom, float4* s_phi) {
+  constexpr bool kMom = (MODE & NZ_MODE_MOMENTS) != 0;
+  constexpr bool kDisp = (MODE & kModeDisp) != 0;
+  constexpr bool kOrig = kMom || kDisp;  // origin in registers
+  constexpr bool kT64 = (MODE & NZ_MODE_TANGENT64) != 0;
+  constexpr unsigned kAll = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  float x = 0.f, y = 0.f, z = 0.f;
+  int label = 0;
+  uint32_t wid = 0;
+  float sig = 1.f;
+  static_assert(!(kOrig && (MODE & NZ_MODE_PHI)), "one of phase sums and origin");
+  float4& phi_sum = s_phi[threadIdx.x];  // phase modes only
+  float4& origin = s_phi[threadIdx.x];   // moment modes only
+  float2& phi_comp = reinterpret_cast<float2*>(s_phi + blockDim.x)[threadIdx.x];
+  int s = live ? s0 : s1;
+  int niter = 0, cell = 0;
+  // start and count of the step cell's primary list (the near list where
+  // there is one), loaded as soon as the cell is known so that the load
+  // overlaps the draw
+  int pstart = 0, pcount = 0;
+  float mx = 0.f, my = 0.f, mz = 0.f;  // centre of the step's cell
+  float jr = 1.0f, jx = 0.0f, jy = 0.0f, jz = 0.0f;
+  // ds depends on the label only; it is recomputed when the label at the
+  // start of a step differs from the one it was computed for
+  int ds_label = 0;
+  float ds = 0.f;
+  int oob = 0;  // bounds-checked build: an index was out of range
+  int lo = 0, hi = 0;  // keys of structure `label`
+  int within = -1;     // index form: record of a sphere that contained the walker (-1: none known)
+  const float dt = J.dt;
+  const bool has_near = (LK ? J.near_idx : static_cast<const void*>(J.near_sph4)) != nullptr;
+  if (live) {
+    const float4 P = J.pos[w];
+    x = P.x; y = P.y; z = P.z;
+    label = __float_as_int(P.w);
+    wid = __float_as_uint(J.org[w].w);
+    if (MODE & NZ_MODE_SIG) sig = J.phi[w].w;
+    if (MODE & NZ_MODE_PHI) {
+      const float4 F = J.phi[w], C = J.comp[w];
+      phi_sum = make_float4(F.x, F.y, F.z, C.x);
+      phi_comp = make_float2(C.y, C.z);
+    }
+    if (kOrig) origin = J.org[w];
+    if (label < 0 || label > J.nstructures) label = J.nstructures;
+    label_bounds<LK>(J, label, lo, hi);
+    ds_label = label;
+    ds = sqrtf(2 * __ldg(J.D + label) * dt);
+    cell = step_cell(J, x, y, z, mx, my, mz);
+    cell_list(J, has_near, cell, pstart, pcount, oob);
+    jump_of(J, wid, s, 0, ds, jx, jy, jz);
+  }
+  while (__any_sync(0xffffffffu, s < s1)) {
+    const bool act = s < s1;
+    float jc = jr;
+    float a = jx * jx + jy * jy + jz * jz;
+    float reach = reach_of(a, jr);
+    // Near list when everything this iteration can touch lies within its
+    // margin of the step's cell: distance from the walker to the cell plus
+    // the reach, with 2 % + 2 nm of slack against rounding
+    // ((dist + reach) * 1.02 + tol + 2 nm <= margin, as dist^2 <= t^2 with
+    // t = near_cut - reach).
+    bool near = false;
+    if (has_near) {
+      const float ex = fmaxf(0.f, __fmaf_rn(-0.5f, J.g.dLx, fabsf(x - mx)));
+      const float ey = fmaxf(0.f, __fmaf_rn(-0.5f, J.g.dLy, fabsf(y - my)));
+      const float ez = fmaxf(0.f, __fmaf_rn(-0.5f, J.g.dLz, fabsf(z - mz)));
+      const float t = J.near_cut - reach;
+      near = t >= 0.f && __fmaf_rn(ex, ex, __fmaf_rn(ey, ey, ez * ez)) <= t * t;
+    }
+    int start = pstart, count = act ? pcount : 0;
+    if (act && has_near && !near) cell_list(J, false, cell, start, count, oob);
+    // A sphere of the walker's structure whose safe ball (nz_cells_safe)
+    // contains the segment's ends, and so all of it: the walker stays inside
+    // that sphere and out of reach of every lower structure's, so it keeps
+    // its label and takes the whole jump, and no list is scanned.  Tried: the
+    // sphere that held the walker longest when its fractions were last
+    // computed.
+    bool deep = false;
+    if (LK != 0 && J.rec_safe && within >= lo && within < hi && near && a >= 1e-8f) {
+      const float4 c = SH ? s_stage[within] : __ldg(J.rec4 + within);
+      const float safe = __ldg(J.rec_safe + within);
+      const float dx = x - c.x, dy = y - c.y, dz = z - c.z;
+      const float ux = __fmaf_rn(jr, jx, dx), uy = __fmaf_rn(jr, jy, dy), uz = __fmaf_rn(jr, jz, dz);
+      deep = fmaxf(__fmaf_rn(dx, dx, __fmaf_rn(dy, dy, dz * dz)), __fmaf_rn(ux, ux, __fmaf_rn(uy, uy, uz * uz))) < safe;
+    }
+    // The collision pass.  Each lane marks its list's near entries 32 at a
+    // time and computes their fractions:
+    //  * packed near lists (the usual case): near_bits_packed;
+    //  * an iteration that needs the full list where near lists are packed (1
+    //    walker in 100): the warp tests that list together, an entry a lane,
+    //    so the others do not wait for a lane's 20 and more entries;
+    //  * lists without packed entries: near_bits.
+    ScanOut r;
+    r.fin = 0.0f;
+    r.fout = kBig;
+    r.any_in = false;
+    bool lower = false;
+    bool more = act && !deep && count > 0;
+    const bool packed = LK != 0 && J.near_pack != nullptr;
+    const bool tiny = a < 1e-8f;  // a jump too short for the filter's arithmetic: every entry is near
+    const float inf = __int_as_float(0x7f800000);
+    const void* list = LK ? (near ? J.near_idx : J.idx) : nullptr;
+    const float4* rec = LK ? J.rec4 : (near ? J.near_sph4 : J.sph4);
+    const int* sid = LK ? nullptr : (near ? J.near_sid : J.sid);
+    const unsigned full0 = packed ? __ballot_sync(kAll, more && !near) : 0u;
+    Reach g;
+    if (!packed || full0) {
+      const float f = 2.0f * jr;
+      g.mx = f * jx;
+      g.my = f * jy;
+      g.mz = f * jz;
+      g.m2 = a * (jr * jr);
+      g.k = -0.5f * rcp_approx(g.m2);
+      g.slack = tiny ? inf : kTol + 2e-3f + 0.02f * reach;
+    }
+    __half2 px, py, pz, ex, ey, ez, len, grow;
+    const uint4* pk = nullptr;
+    if (packed) {
+      const float ir = rsqrt_approx(fmaxf(a, 1e-30f));
+      px = __float2half2_rn(x - mx);
+      py = __float2half2_rn(y - my);
+      pz = __float2half2_rn(z - mz);
+      ex = __float2half2_rn(jx * ir);
+      ey = __float2half2_rn(jy * ir);
+      ez = __float2half2_rn(jz * ir);
+      len = __float2half2_rn(reach);
+      grow = __float2half2_rn(tiny ? inf : 0.02f * reach);
+      pk = J.near_pack + ((start + cell + 1) >> 1);
+    }
+    for (int base = 0; __any_sync(kAll, more); base += 32) {
+      uint32_t bits = 0u;
+      if (more) {
+        const int n = min(32, count - base);
+        if (!packed)
+          bits = near_bits<LK, SH>(list, rec, sid, start + base, n, hi, J.S, oob, g, x, y, z);
+        else if (near)
+          bits = near_bits_packed(pk + (base >> 1), (n + 1) >> 1, px, py, pz, ex, ey, ez, len, grow) &
+                 (((1u << ((n + 1) >> 1)) - 1u) | (((1u << (n >> 1)) - 1u) << 16));
+      }
+      unsigned full = full0 ? __ballot_sync(kAll, more && !near) : 0u;
+      while (full) {
+        const int o = __ffs(full) - 1;
+        full &= full - 1;
+        Reach go;
+        go.mx = __shfl_sync(kAll, g.mx, o);
+        go.my = __shfl_sync(kAll, g.my, o);
+        go.mz = __shfl_sync(kAll, g.mz, o);
+        go.m2 = __shfl_sync(kAll, g.m2, o);
+        go.k = __shfl_sync(kAll, g.k, o);
+        go.slack = __shfl_sync(kAll, g.slack, o);
+        const float xo = __shfl_sync(kAll, x, o), yo = __shfl_sync(kAll, y, o), zo = __shfl_sync(kAll, z, o);
+        const int so = __shfl_sync(kAll, start, o), no = __shfl_sync(kAll, count, o), ho = __shfl_sync(kAll, hi, o);
+        // lane's entry: the one whose mark is bit `lane` (bit_entry)
+        const int i = base + bit_entry(lane);
+        bool yes = false;
+        int bad = 0;
+        if (i < no) {
+          int key;
+          float4 c;
+          entry<LK, SH>(J.idx, J.rec4, nullptr, so + i, J.S, bad, key, c);
+          yes = key < ho && is_near(go, xo, yo, zo, c);
+        }
+        const unsigned m = __ballot_sync(kAll, yes);
+        if (kCheckBounds) bad = __any_sync(kAll, bad);
+        if (lane == o) {
+          bits = m;
+          oob |= bad;
+        }
+      }
+      if (bits)
+        fractions<LK, kT64, SH>(bits, list, rec, sid, start + base, lo, hi, x, y, z, a, jx, jy, jz, J.S, oob, r, lower,
+                                within);
+      more = more && base + 32 < count;
+    }
+    if (!act) continue;
+    niter++;
+    if (deep) {
+      r.any_in = true;
+      r.fin = jr;
+    }
+    // the label carried from the previous iteration holds when no sphere of a
+    // lower structure contains the walker and, outside the box, one of its own does
+    if (lower || (label < J.nstructures && !r.any_in)) {
+      label = label_of<LK, SH>(list, rec, sid, J.rec_sid, start, count, J.nstructures, x, y, z, J.S, oob);
+      if (kCheckBounds && (label < 0 || label > J.nstructures)) {
+        oob = 1;
+        label = J.nstructures;
+      }
+      label_bounds<LK>(J, label, lo, hi);
+      if (niter == 1) {  // the first draw's length depends on the label
+        ds = sqrtf(2 * __ldg(J.D + label) * dt);
+        ds_label = label;
+        jump_of(J, wid, s, 0, ds, jx, jy, jz);
+        a = jx * jx + jy * jy + jz * jz;
+      }
+      // the full list: the near one was chosen for the old reach
+      int fs, fc;
+      cell_list(J, false, cell, fs, fc, oob);
+      scan_lane<LK, kT64, SH>(LK ? J.idx : nullptr, LK ? J.rec4 : J.sph4, LK ? nullptr : J.sid, fs, fc, lo, hi, x, y,
+                              z, a, jx, jy, jz, J.S, oob, r);
+    }
+    jc = ref_min(jc, r.any_in ? r.fin : kBig);
+    jc = ref_min(jc, r.fout);
+    x += jc * jx;
+    y += jc * jy;
+    z += jc * jz;
+    // the next draw: the scatter draw of this step, or the first draw of the
+    // next one; every iteration ends with one or the other, so one call site
+    // serves all lanes of the warp
+    // (the k-th iteration's scatter draw is draw k)
+    int next_step = s, next_draw = niter;
+    if (jc < jr) {
+      jr = sqrtf(ref_max(0, jr * jr - jc * jc));
+      if (MODE & NZ_MODE_SIG) sig *= t2_decay(-jc * jc * dt / __ldg(J.T2 + label));
+    } else {
+      jr -= jc;
+      if (MODE & NZ_MODE_SIG) sig *= t2_decay(-jc * dt / __ldg(J.T2 + label));
+    }
+    if (!((jr > kTol) && (niter < kMaxIter))) {
+      if (niter >= kMaxIter && jr > kTol) {
+        float4* c = J.comp + w;
+        c->w = __int_as_float(__float_as_int(c->w) | kFlagIterCap);
+      }
+      float fx, fy, fz, kx, ky, kz;
+      if (MODE & NZ_MODE_PHI) {
+        const float4 F = phi_sum;
+        const float2 C = phi_comp;
+        fx = F.x; fy = F.y; fz = F.z; kx = F.w; ky = C.x; kz = C.y;
+        const float G = __ldg(J.G + s);
+        kahan_add(fx, kx, G * x);
+        kahan_add(fy, ky, G * y);
+        kahan_add(fz, kz, G * z);
+      }
+      const float Lx = J.g.Lx, Ly = J.g.Ly, Lz = J.g.Lz;
+      if (fabsf(x) > Lx / 2 || fabsf(y) > Ly / 2 || fabsf(z) > Lz / 2) {  // rare: a wrap
+        const float Ga = (MODE & NZ_MODE_PHI) ? __ldg(J.Garea + s) : 0.0f;
+        float4 O = kOrig ? origin : J.org[w];
+        if (x < -Lx / 2) {
+          x += Lx; O.x += Lx;
+          if (MODE & NZ_MODE_PHI) kahan_add(fx, kx, Lx * Ga);
+        } else if (x > Lx / 2) {
+          x -= Lx; O.x -= Lx;
+          if (MODE & NZ_MODE_PHI) kahan_add(fx, kx, -(Lx * Ga));
+        }
+        if (y < -Ly / 2) {
+          y += Ly; O.y += Ly;
+          if (MODE & NZ_MODE_PHI) kahan_add(fy, ky, Ly * Ga);
+        } else if (y > Ly / 2) {
+          y -= Ly; O.y -= Ly;
+          if (MODE & NZ_MODE_PHI) kahan_add(fy, ky, -(Ly * Ga));
+        }
+        if (z < -Lz / 2) {
+          z += Lz; O.z += Lz;
+          if (MODE & NZ_MODE_PHI) kahan_add(fz, kz, Lz * Ga);
+        } else if (z > Lz / 2) {
+          z -= Lz; O.z -= Lz;
+          if (MODE & NZ_MODE_PHI) kahan_add(fz, kz, -(Lz * Ga));
+        }
+        if (kOrig) origin = O;
+        else J.org[w] = O;
+      }
+      if (MODE & NZ_MODE_PHI) {
+        phi_sum = make_float4(fx, fy, fz, kx);
+        phi_comp = make_float2(ky, kz);
+      }
+      if (kDisp) {  // coalesced across the warp's walkers of one step
+        const size_t N = size_t(J.nwalkers);
+        float* d = J.disp + size_t(s - s0) * 3 * N;
+        const float4 O = origin;
+        d[w] = x - O.x;
+        d[N + w] = y - O.y;
+        d[2 * N + w] = z - O.z;
+      }
+      if (kMom) {  // nz_moments' terms: float displacement, squared in FP64
+        const float4 O = origin;
+        const double ex = double(x - O.x), ey = double(y - O.y), ez = double(z - O.z);
+        double* m = s_mom + 6 * (s - s0);
+        const double ex2 = ex * ex, ey2 = ey * ey, ez2 = ez * ez;
+        atomicAdd(m + 0, ex2);
+        atomicAdd(m + 1, ey2);
+        atomicAdd(m + 2, ez2);
+        atomicAdd(m + 3, ex2 * ex2);
+        atomicAdd(m + 4, ey2 * ey2);
+        atomicAdd(m + 5, ez2 * ez2);
+      }
+      s++;
+      niter = 0;
+      jr = 1.0f;
+      next_step = s;
+      next_draw = 0;
+      if (label != ds_label) {
+        ds = sqrtf(2 * __ldg(J.D + label) * dt);
+        ds_label = label;
+      }
+      cell = step_cell(J, x, y, z, mx, my, mz);
+      cell_list(J, has_near, cell, pstart, pcount, oob);
+    }
+    if (s < s1) jump_of(J, wid, next_step, next_draw, ds, jx, jy, jz);
+  }
+  if (!live) return;
+  J.pos[w] = make_float4(x, y, z, __int_as_float(label));
+  if (kOrig) J.org[w] = origin;
+  if (MODE & NZ_MODE_PHI) {
+    const float4 F = phi_sum;
+    J.phi[w] = make_float4(F.x, F.y, F.z, (MODE & NZ_MODE_SIG) ? sig : J.phi[w].w);
+    float4* c = J.comp + w;
+    *c = make_float4(F.w, phi_comp.x, phi_comp.y, c->w);
+  } else if (MODE & NZ_MODE_SIG) {
+    J.phi[w].w = sig;
+  }
+  if (kCheckBounds && oob) {
+    float4* c = J.comp + w;
+    c->w = __int_as_float(__float_as_int(c->w) | kFlagBounds);
+  }
+}
+
+// Steps [s0, s1) of walker w, by a lane on its own: lists without packed
+// entries (on full lists of 25 entries, 1e8 walker-steps: 11.0 ms so, 11.7
+// through walk_warp, record lists 12.3 and 14.0).  Registers hold position, label, Phi and its
 // compensation and the step's jump; the origin (spins0) and the flag word stay
 // in memory and are updated in place on the rare wrap / iteration-cap events
 // (except with moments, which read the origin every step).
@@ -279,8 +777,8 @@ __device__ __forceinline__ void walk_one(const JobDev& J, int w, int s0, int s1,
     x0 = O.x; y0 = O.y; z0 = O.z;
   }
   if (label < 0 || label > J.nstructures) label = J.nstructures;
-  int lo = 0, hi = 0;  // index form: structure `label`'s records
-  if (LK) label_bounds(J, label, lo, hi);
+  int lo, hi;  // keys of structure `label`
+  label_bounds<LK>(J, label, lo, hi);
 
   const float dt = J.dt;
   const bool has_near = (LK ? J.near_idx : static_cast<const void*>(J.near_sph4)) != nullptr;
@@ -290,7 +788,7 @@ __device__ __forceinline__ void walk_one(const JobDev& J, int w, int s0, int s1,
   // there is one), loaded as soon as the cell is known so that the load
   // overlaps the draw
   int pstart = 0, pcount = 0;
-  float lox = 0.f, loy = 0.f, loz = 0.f;  // low corner of the step's cell
+  float mx = 0.f, my = 0.f, mz = 0.f;  // centre of the step's cell
   float jr = 1.0f, jx = 0.0f, jy = 0.0f, jz = 0.0f;
   // ds depends on the label only; it is recomputed when the label at the
   // start of a step differs from the one it was computed for
@@ -298,7 +796,7 @@ __device__ __forceinline__ void walk_one(const JobDev& J, int w, int s0, int s1,
   float ds = sqrtf(2 * __ldg(J.D + label) * dt);
   int oob = 0;  // bounds-checked build: an index was out of range
   if (s < s1) {
-    cell = step_cell(J, x, y, z, lox, loy, loz);
+    cell = step_cell(J, x, y, z, mx, my, mz);
     cell_list(J, has_near, cell, pstart, pcount, oob);
     jump_of(J, wid, s, 0, ds, jx, jy, jz);
     draw = 1;
@@ -315,9 +813,9 @@ __device__ __forceinline__ void walk_one(const JobDev& J, int w, int s0, int s1,
     // t = near_cut - reach).
     bool near = false;
     if (has_near) {
-      const float ex = fmaxf(0.f, fmaxf(lox - x, x - (lox + J.g.dLx)));
-      const float ey = fmaxf(0.f, fmaxf(loy - y, y - (loy + J.g.dLy)));
-      const float ez = fmaxf(0.f, fmaxf(loz - z, z - (loz + J.g.dLz)));
+      const float ex = fmaxf(0.f, __fmaf_rn(-0.5f, J.g.dLx, fabsf(x - mx)));
+      const float ey = fmaxf(0.f, __fmaf_rn(-0.5f, J.g.dLy, fabsf(y - my)));
+      const float ez = fmaxf(0.f, __fmaf_rn(-0.5f, J.g.dLz, fabsf(z - mz)));
       const float t = J.near_cut - reach;
       near = t >= 0.f && ex * ex + ey * ey + ez * ez <= t * t;
     }
@@ -335,7 +833,7 @@ __device__ __forceinline__ void walk_one(const JobDev& J, int w, int s0, int s1,
         oob = 1;
         label = J.nstructures;
       }
-      if (LK) label_bounds(J, label, lo, hi);
+      label_bounds<LK>(J, label, lo, hi);
       if (niter == 1) {  // the first draw's length depends on the label
         ds = sqrtf(2 * __ldg(J.D + label) * dt);
         ds_label = label;
@@ -436,7 +934,7 @@ __device__ __forceinline__ void walk_one(const JobDev& J, int w, int s0, int s1,
         ds = sqrtf(2 * __ldg(J.D + label) * dt);
         ds_label = label;
       }
-      cell = step_cell(J, x, y, z, lox, loy, loz);
+      cell = step_cell(J, x, y, z, mx, my, mz);
       cell_list(J, has_near, cell, pstart, pcount, oob);
     }
     if (s < s1) jump_of(J, wid, next_step, next_draw, ds, jx, jy, jz);
@@ -456,18 +954,21 @@ __device__ __forceinline__ void walk_one(const JobDev& J, int w, int s0, int s1,
 
 // One work item: walkers [first, first + count) of job J, steps [step0, step1)
 // clamped to the job's protocol.
-template <int MODE, int LK, bool SH>
+template <int MODE, int LK, bool SH, bool WARP>
 __device__ __forceinline__ void run_item(const JobDev& J, int first, int count, int step0, int step1, double* s_mom,
-                                         int flags = 0) {
+                                         float4* s_phi, int flags = 0, int lanes = 32) {
   const int s0 = step0 + J.step_offset, s1 = min(step1 + J.step_offset, J.nsteps);
   if (MODE & NZ_MODE_MOMENTS) {
     for (int i = threadIdx.x; i < kMomentSteps * 6; i += blockDim.x) s_mom[i] = 0.0;
     __syncthreads();
   }
-  if (threadIdx.x < count && s0 < s1) {
-    walk_one<MODE, LK, SH>(J, first + threadIdx.x, s0, s1, s_mom);
-    if (flags) {
-      float4* c = J.comp + first + threadIdx.x;
+  const int slot = int(threadIdx.x >> 5) * lanes + int(threadIdx.x & 31);
+  const bool live = int(threadIdx.x & 31) < lanes && slot < count && s0 < s1;
+  if (WARP ? __any_sync(0xffffffffu, live) : live) {
+    if constexpr (WARP) walk_warp<MODE, LK, SH>(J, live, first + slot, s0, s1, s_mom, s_phi);
+    else walk_one<MODE, LK, SH>(J, first + slot, s0, s1, s_mom);
+    if (live && flags) {
+      float4* c = J.comp + first + slot;
       c->w = __int_as_float(__float_as_int(c->w) | flags);
     }
   }
@@ -520,7 +1021,7 @@ __device__ __forceinline__ void stage_records(uint32_t bar, const float4* src, u
 }
 
 // Work items are CTAs' worth of walkers of one job.  SINGLE: one job passed by
-// value, item i = walkers [i*T, i*T + T).  Otherwise jobs and items come from
+// value, stage_cap walkers a warp, item i = the i-th CTA's worth of them.  Otherwise jobs and items come from
 // device arrays; with queue != null the grid is persistent and each CTA takes
 // items from *queue until none is left.
 // STAGE (batched, index lists): a job whose S records fit in stage_cap
@@ -534,11 +1035,13 @@ __device__ __forceinline__ void stage_records(uint32_t bar, const float4* src, u
 #else
 #define NZ_FUSED_BOUNDS __launch_bounds__(kFusedMaxThreads, kFusedMinBlocks)
 #endif
-template <int MODE, int LK, bool SINGLE, bool STAGE>
+enum : int { kBatch, kSingle, kSinglePacked };  // kinds of launch: one job with or without packed near lists
+template <int MODE, int LK, int KIND, bool STAGE>
 __global__ void NZ_FUSED_BOUNDS
     walk_fused_kernel(const __grid_constant__ JobDev single, const nz_job* __restrict__ jobs,
                       const nz_item* __restrict__ items, int n_items, int step0, int step1, int* queue,
                       int stage_cap) {
+  constexpr bool SINGLE = KIND != kBatch;
   static_assert(!STAGE || (!SINGLE && LK != 0), "staging is for batched index-list walks");
   __shared__ int s_item;
   __shared__ double s_mom[(MODE & NZ_MODE_MOMENTS) ? kMomentSteps * 6 : 1];
@@ -546,6 +1049,7 @@ __global__ void NZ_FUSED_BOUNDS
   __shared__ __align__(8) uint64_t s_bar;
   __shared__ const float4* s_staged;  // the records now in s_stage (thread 0's bookkeeping)
   __shared__ int s_use, s_broken, s_pending;
+  float4* const s_phi = s_stage + (STAGE ? stage_cap : 0);
   uint32_t phase = 0;  // parity of the barrier phase the next copy completes
   if (STAGE) {
     if (threadIdx.x == 0) {
@@ -570,9 +1074,11 @@ __global__ void NZ_FUSED_BOUNDS
       return;
     }
     if (SINGLE) {
-      const int first = it * int(blockDim.x);
-      const int count = min(int(blockDim.x), single.nwalkers - first);
-      run_item<MODE, LK, false>(single, first, count, step0, step1, s_mom);
+      const int lanes = stage_cap;  // walkers a warp
+      const int per = int(blockDim.x >> 5) * lanes;
+      const int first = it * per;
+      const int count = min(per, single.nwalkers - first);
+      run_item<MODE, LK, false, KIND == kSinglePacked>(single, first, count, step0, step1, s_mom, s_phi, 0, lanes);
     } else {
       // every thread of the CTA works on the same job: its descriptor lives
       // in shared memory, not in each thread's registers
@@ -620,10 +1126,10 @@ __global__ void NZ_FUSED_BOUNDS
             }
           }
         }
-        if (use) run_item<MODE, LK, true>(s_job, wi.first, wi.count, step0, step1, s_mom);
-        else run_item<MODE, LK, false>(s_job, wi.first, wi.count, step0, step1, s_mom, flags);
+        if (use) run_item<MODE, LK, true, true>(s_job, wi.first, wi.count, step0, step1, s_mom, s_phi);
+        else run_item<MODE, LK, false, LK != 0>(s_job, wi.first, wi.count, step0, step1, s_mom, s_phi, flags);
       } else {
-        run_item<MODE, LK, false>(s_job, wi.first, wi.count, step0, step1, s_mom);
+        run_item<MODE, LK, false, LK != 0>(s_job, wi.first, wi.count, step0, step1, s_mom, s_phi);
       }
       __syncthreads();
     }
@@ -696,6 +1202,7 @@ __host__ __device__ JobDev make_job(const nz_substrate& sub, const float* G, con
   j.idLy = 1.0f / sub.grid.dLy;
   j.idLz = 1.0f / sub.grid.dLz;
   j.nstructures = sub.nstructures;
+  j.ncell = sub.grid.nx * sub.grid.ny * sub.grid.nz;
   j.sph4 = reinterpret_cast<const float4*>(sub.cell_sph4);
   j.sid = sub.cell_sid;
   j.cell_start = sub.cell_start;
@@ -705,6 +1212,11 @@ __host__ __device__ JobDev make_job(const nz_substrate& sub, const float* G, con
   j.near_start = sub.near_start;
   j.near_count = sub.near_count;
   j.near_sph4 = reinterpret_cast<const float4*>(sub.near_sph4);
+  // packed near entries: the pairs, then the squared safe radius of every record
+  j.near_pack = (sub.idx_bytes & NZ_NEAR_PACKED) && sub.near_idx ? reinterpret_cast<const uint4*>(sub.near_sph4)
+                                                                 : nullptr;
+  j.rec_safe = j.near_pack ? reinterpret_cast<const float*>(j.near_pack + pack_pairs(sub.near_items, j.ncell))
+                           : nullptr;
   j.near_sid = sub.near_sid;
   j.idx = sub.idx_bytes ? sub.cell_idx : nullptr;
   j.near_idx = sub.idx_bytes ? sub.near_idx : nullptr;
@@ -712,7 +1224,6 @@ __host__ __device__ JobDev make_job(const nz_substrate& sub, const float* G, con
   j.rec_sid = sub.rec_sid;
   j.sid_start = sub.sid_start;
   j.S = sub.S;
-  j.ncell = sub.grid.nx * sub.grid.ny * sub.grid.nz;
   j.n_items = sub.n_items;
   j.near_items = sub.near_items;
   j.D = sub.D;
@@ -738,22 +1249,31 @@ __host__ __device__ JobDev make_job(const nz_substrate& sub, const float* G, con
 // setting its attributes: the largest allowed size (once per device) and a
 // carveout that leaves room for the CTAs the register budget allows at this
 // CTA size, the rest staying L1.
+// Shared memory carveout (percent) of the unstaged walk: what the CTAs that
+// the register budget allows need (and 1 KB each that the system takes); the
+// rest stays L1, which the lists and records live in.
+template <int MODE>
+constexpr int fused_carveout() {
+  constexpr size_t need = kFusedMinBlocks * phi_bytes<MODE>(kFusedMaxThreads) + 2 * kFusedMinBlocks * 1400;
+  return phi_bytes<MODE>(32) ? int((100 * need + kSmemPerSm - 1) / kSmemPerSm) : 0;
+}
+
 template <int MODE, int LK>
 size_t stage_setup(int stage_cap, int threads) {
-  const size_t bytes = size_t(stage_cap) * 16;
+  const size_t bytes = size_t(stage_cap) * 16 + phi_bytes<MODE>(threads);
   if (LK == 0 || stage_cap <= 0) return 0;
   int dev = 0;
   if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < kMaxDevices) {
     static std::once_flag once[kMaxDevices];
     std::call_once(once[dev], [] {
-      cudaFuncSetAttribute(walk_fused_kernel<MODE, LK, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           kMaxStageRecords * 16);
+      cudaFuncSetAttribute(walk_fused_kernel<MODE, LK, kBatch, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           kMaxStageRecords * 16 + int(phi_bytes<MODE>(kFusedMaxThreads)));
     });
   }
   const int ctas = std::max(1, kFusedMinBlocks * kFusedMaxThreads / threads);
   const size_t need = size_t(ctas) * (bytes + 2048);
   const int pct = int(std::min<size_t>(100, (100 * need + kSmemPerSm - 1) / kSmemPerSm));
-  cudaFuncSetAttribute(walk_fused_kernel<MODE, LK, false, true>, cudaFuncAttributePreferredSharedMemoryCarveout, pct);
+  cudaFuncSetAttribute(walk_fused_kernel<MODE, LK, kBatch, true>, cudaFuncAttributePreferredSharedMemoryCarveout, pct);
   return bytes;
 }
 
@@ -767,26 +1287,38 @@ void launch_mode(const JobDev& single, const nz_job* jobs, const nz_item* items,
   if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < kMaxDevices) {
     static std::once_flag once[kMaxDevices];
     std::call_once(once[dev], [] {
-      cudaFuncSetAttribute(walk_fused_kernel<MODE, LK, false, false>, cudaFuncAttributePreferredSharedMemoryCarveout,
+      cudaFuncSetAttribute(walk_fused_kernel<MODE, LK, kBatch, false>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                           LK ? fused_carveout<MODE>() : 0);
+      cudaFuncSetAttribute(walk_fused_kernel<MODE, LK, kSingle, false>, cudaFuncAttributePreferredSharedMemoryCarveout,
                            0);
-      cudaFuncSetAttribute(walk_fused_kernel<MODE, LK, true, false>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                           0);
+      if constexpr (LK != 0)
+        cudaFuncSetAttribute(walk_fused_kernel<MODE, LK, kSinglePacked, false>,
+                             cudaFuncAttributePreferredSharedMemoryCarveout, fused_carveout<MODE>());
     });
   }
   if constexpr (LK != 0) {
     if (jobs && stage_cap > 0) {
       const size_t smem = stage_setup<MODE, LK>(stage_cap, threads);
-      walk_fused_kernel<MODE, LK, false, true>
+      walk_fused_kernel<MODE, LK, kBatch, true>
           <<<grid, threads, smem, st>>>(single, jobs, items, n_items, step0, step1, queue, stage_cap);
       return;
     }
   }
-  if (jobs)
-    walk_fused_kernel<MODE, LK, false, false>
-        <<<grid, threads, 0, st>>>(single, jobs, items, n_items, step0, step1, queue, 0);
-  else
-    walk_fused_kernel<MODE, LK, true, false>
-        <<<grid, threads, 0, st>>>(single, jobs, items, n_items, step0, step1, queue, 0);
+  const size_t bytes = phi_bytes<MODE>(threads);
+  if (jobs) {
+    walk_fused_kernel<MODE, LK, kBatch, false>
+        <<<grid, threads, LK ? bytes : 0, st>>>(single, jobs, items, n_items, step0, step1, queue, 0);
+    return;
+  }
+  if constexpr (LK != 0) {
+    if (single.near_pack) {
+      walk_fused_kernel<MODE, LK, kSinglePacked, false>
+          <<<grid, threads, bytes, st>>>(single, jobs, items, n_items, step0, step1, queue, stage_cap);
+      return;
+    }
+  }
+  walk_fused_kernel<MODE, LK, kSingle, false>
+      <<<grid, threads, 0, st>>>(single, jobs, items, n_items, step0, step1, queue, stage_cap);
 }
 
 template <int LK>
@@ -817,7 +1349,9 @@ int launch_lk(int mode, const JobDev& single, const nz_job* jobs, const nz_item*
 int launch_fused(int mode, int lk, const JobDev& single, const nz_job* jobs, const nz_item* items, int n_items,
                  int step0, int step1, int* queue, int grid, int threads, cudaStream_t st, int stage_cap) {
   switch (lk) {
-    case 0: return launch_lk<0>(mode, single, jobs, items, n_items, step0, step1, queue, grid, threads, 0, st);
+    case 0:
+      return launch_lk<0>(mode, single, jobs, items, n_items, step0, step1, queue, grid, threads, jobs ? 0 : stage_cap,
+                          st);
     case 2:
       return launch_lk<2>(mode, single, jobs, items, n_items, step0, step1, queue, grid, threads, stage_cap, st);
     case 4:
@@ -831,12 +1365,12 @@ cudaError_t occupancy_mode(int threads, int stage_cap, int* blocks_per_sm) {
   if constexpr (LK != 0) {
     if (stage_cap > 0) {
       const size_t smem = stage_setup<MODE, LK>(stage_cap, threads);
-      return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, walk_fused_kernel<MODE, LK, false, true>,
+      return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, walk_fused_kernel<MODE, LK, kBatch, true>,
                                                            threads, smem);
     }
   }
-  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, walk_fused_kernel<MODE, LK, false, false>,
-                                                       threads, 0);
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, walk_fused_kernel<MODE, LK, kBatch, false>,
+                                                       threads, LK ? phi_bytes<MODE>(threads) : 0);
 }
 
 template <int LK>

@@ -165,6 +165,18 @@ class DeviceSubstrate:
                                         self.idx_bytes, _stream()), "nz_cells_index")
         return idx
 
+    def _pack(self, start, count, idx, n, margin):
+        """The packed near entries of index lists (nz_cells_pack); None for
+        cells too large for it."""
+        if max(self.grid.dLx, self.grid.dLy, self.grid.dLz) > 1e4:
+            return None
+        lib = L.load()
+        pack = torch.empty(int(lib.nz_cells_pack_bytes(n, self.ncell, self.S)), dtype=torch.uint8, device=_dev())
+        L.check(lib.nz_cells_pack(_p(self.rec4), _p(self.rec_sid), self.S, _p(idx), self.idx_bytes, _p(start),
+                                  _p(count), n, _p(self.cell_idx), _p(self.cell_start), _p(self.cell_count),
+                                  L.byref(self.grid), np.float32(margin), _p(pack), _stream()), "nz_cells_pack")
+        return pack
+
     def _build_cells(self, margin: float | None = None, store: bool = True, rounded: bool = False):
         """Member lists with the reference's box test (margin: jump_tol by
         default); rounded: the near lists' Euclidean test (nz_cells_*_round)."""
@@ -208,7 +220,8 @@ class DeviceSubstrate:
         self.near_n = n
         if self.idx_bytes:
             self.near_margin = margin
-            self.near = (st, ct, it, None, None, self._index(st, ct, it, n))
+            idx = self._index(st, ct, it, n)
+            self.near = (st, ct, it, self._pack(st, ct, idx, n, margin), None, idx)
             return
         sph4 = torch.empty((max(n, 1), 4), dtype=torch.float32, device=dev)
         sid = torch.empty(max(n, 1), dtype=torch.int32, device=dev)
@@ -268,13 +281,14 @@ class DeviceSubstrate:
                         ptr(self.cell_sid), self.D.data_ptr(), self.T2.data_ptr())
         s.n_items = int(self.n_items)
         if self.near is not None:
-            st, ct, _, sph4, sid, nidx = self.near
+            st, ct, _, sph4, sid, nidx = self.near  # sph4: records, or the packed entries of index lists
             s.near_margin = self.near_margin
             s.near_start, s.near_count = st.data_ptr(), ct.data_ptr()
             s.near_sph4, s.near_sid, s.near_idx = ptr(sph4), ptr(sid), ptr(nidx)
             s.near_items = int(self.near_n)
         if self.idx_bytes:
-            s.idx_bytes, s.cell_idx = self.idx_bytes, self.cell_idx.data_ptr()
+            packed = L.NEAR_PACKED if self.near is not None and self.near[3] is not None else 0
+            s.idx_bytes, s.cell_idx = self.idx_bytes + packed, self.cell_idx.data_ptr()
             s.rec4, s.rec_sid, s.sid_start = self.rec4.data_ptr(), self.rec_sid.data_ptr(), self.sid_start.data_ptr()
         return s
 
