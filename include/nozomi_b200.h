@@ -242,14 +242,12 @@ int nz_cells_index(const int* items, int n_items, const int* perm, int S, const 
  * near lists are taken).  After the pairs, a squared safe radius per record:
  * a walker of the record's structure whose segment stays that close to the
  * record's centre meets no sphere.  idx, start, count: the near lists, laid
- * out without gaps (start the exclusive scan of count); full_*: the cell
- * lists.  pack: nz_cells_pack_bytes(n_items, ncell, S) bytes, 16-byte
+ * out without gaps (start the exclusive scan of count).  pack: nz_cells_pack_bytes(n_items, ncell, S) bytes, 16-byte
  * aligned; nz_substrate.near_items must then be n_items.  Grids with a cell
  * edge above 1e4 um are refused. */
 size_t nz_cells_pack_bytes(int n_items, int ncell, int S);
 int nz_cells_pack(const float* rec4, const int* rec_sid, int S, const void* idx, int idx_bytes, const int* start,
-                  const int* count, int n_items, const void* full_idx, const int* full_start, const int* full_count,
-                  const nz_grid* grid, float margin, void* pack, void* stream);
+                  const int* count, int n_items, const nz_grid* grid, float margin, void* pack, void* stream);
 
 /* ---- a12: substrate ingestion on the device — split_matrix_to_list
  * (utils/common_utils.py:41-55) and createBoundaryZ / create_pad

@@ -89,7 +89,7 @@ SIGNATURES = {
     "nz_cells_gather": (_i, [_P, _i, _P, _i, _P, _P, _i, _P, _P, _P]),
     "nz_cells_index": (_i, [_P, _i, _P, _i, _P, _P, _i, _P, _i, _P]),
     "nz_cells_pack_bytes": (ctypes.c_size_t, [_i, _i, _i]),
-    "nz_cells_pack": (_i, [_P, _P, _i, _P, _i, _P, _P, _i, _P, _P, _P, _P, _f, _P, _P]),
+    "nz_cells_pack": (_i, [_P, _P, _i, _P, _i, _P, _P, _i, _P, _f, _P, _P]),
     "nz_collide_scratch_bytes": (ctypes.c_size_t, [_i, _P]),
     "nz_collide_cells": (_i, [_P, _P, _i, _P, _P, _P, ctypes.c_size_t, _P]),
     "nz_collide_pairs": (_i, [_P, _P, _P, _i, _P, _f, _P, _i, _P, _i, _P, _P, ctypes.c_size_t, _P]),

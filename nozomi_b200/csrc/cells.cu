@@ -706,40 +706,38 @@ __global__ void index_fill_kernel(const int* __restrict__ items, int n, const in
 // E is their sum and 15 % more (10 nm for r = 1 um, 0.5 um cells and margin).
 // Spheres that half precision holds badly (R above 100 um, centres beyond
 // 200 um) get R = inf: always near.
-__device__ __forceinline__ void pack_entry(float4 c, double ox, double oy, double oz, double h, double M, __half* v) {
-  const double x = double(c.x) - ox, y = double(c.y) - oy, z = double(c.z) - oz;
-  const double u = 1.0 / 2048, rho = double(c.w) + double(kTol), m = h + 2 * M + rho;
-  const double E = 1.15 * u * (3 * m + 9 * M + 4 * rho + 5.5 * M * M / rho);
-  const double R = double(c.w) * (1.0 + 5e-5) + double(kTol) + 2e-3 + E;
-  const bool fits = R <= 100.0 && fabs(x) <= 200.0 && fabs(y) <= 200.0 && fabs(z) <= 200.0;
-  v[0] = __float2half_rn(fits ? float(x) : 0.0f);
-  v[1] = __float2half_rn(fits ? float(y) : 0.0f);
-  v[2] = __float2half_rn(fits ? float(z) : 0.0f);
-  v[3] = fits ? __float2half_ru(__double2float_ru(R)) : __ushort_as_half(0x7c00);
+__device__ __forceinline__ void pack_entry(float4 c, float ox, float oy, float oz, float h, float M, __half* v) {
+  const float x = c.x - ox, y = c.y - oy, z = c.z - oz;  // single precision: its rounding is in the 15 %
+  const float u = 1.0f / 2048, rho = c.w + kTol, m = h + 2 * M + rho;
+  const float E = 1.15f * u * (3 * m + 9 * M + 4 * rho + 5.5f * M * M / rho);
+  const float R = (c.w * 1.00005f + (kTol + 2e-3f) + E) * 1.000001f;
+  const bool fits = R <= 100.0f && fabsf(x) <= 200.0f && fabsf(y) <= 200.0f && fabsf(z) <= 200.0f;
+  v[0] = __float2half_rn(fits ? x : 0.0f);
+  v[1] = __float2half_rn(fits ? y : 0.0f);
+  v[2] = __float2half_rn(fits ? z : 0.0f);
+  v[3] = fits ? __float2half_ru(R) : __ushort_as_half(0x7c00);
 }
 
+// Eight lanes a cell, a pair each, so that entries are read and pairs written
+// by lines.
 template <typename T>
-__global__ void cells_pack_kernel(const float4* __restrict__ rec4, const T* __restrict__ idx,
-                            const int* __restrict__ start, const int* __restrict__ count, Grid g, double h, double M,
-                            uint4* __restrict__ pack) {
+__global__ void __launch_bounds__(256) cells_pack_kernel(const float4* __restrict__ rec4, const T* __restrict__ idx,
+                                                         const int* __restrict__ start,
+                                                         const int* __restrict__ count, Grid g, float h, float M,
+                                                         uint4* __restrict__ pack) {
   const int nx = int(g.nLx), ny = int(g.nLy), ncell = nx * ny * int(g.nLz);
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  const int c = int((blockIdx.x * size_t(blockDim.x) + threadIdx.x) >> 3), lane = threadIdx.x & 7;
   if (c >= ncell) return;
   const int n = count[c], s = start[c];
-  // the cell's centre as the walk forms it (step_cell's low corner plus half an edge)
-  const double ox = double(float(c % nx) * g.dLx - g.Lx / 2) + 0.5 * g.dLx;
-  const double oy = double(float((c / nx) % ny) * g.dLy - g.Ly / 2) + 0.5 * g.dLy;
-  const double oz = double(float(c / (nx * ny)) * g.dLz - g.Lz / 2) + 0.5 * g.dLz;
+  // the cell's centre as the walk forms it (step_cell)
+  const float ox = __fmaf_rn(float(c % nx), g.dLx, 0.5f * (g.dLx - g.Lx));
+  const float oy = __fmaf_rn(float((c / nx) % ny), g.dLy, 0.5f * (g.dLy - g.Ly));
+  const float oz = __fmaf_rn(float(c / (nx * ny)), g.dLz, 0.5f * (g.dLz - g.Lz));
   uint4* out = pack + ((s + c + 1) >> 1);
-  for (int i = 0; i < n; i += 2) {
+  for (int i = 2 * lane; i < n; i += 16) {
     __half a[4], b[4];
     pack_entry(__ldg(rec4 + int(idx[s + i])), ox, oy, oz, h, M, a);
-    if (i + 1 < n) {
-      pack_entry(__ldg(rec4 + int(idx[s + i + 1])), ox, oy, oz, h, M, b);
-    } else {
-#pragma unroll
-      for (int k = 0; k < 4; ++k) b[k] = a[k];
-    }
+    pack_entry(__ldg(rec4 + int(idx[s + min(i + 1, n - 1)])), ox, oy, oz, h, M, b);
     uint32_t w[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) w[k] = uint32_t(__half_as_ushort(a[k])) | (uint32_t(__half_as_ushort(b[k])) << 16);
@@ -752,45 +750,58 @@ __global__ void cells_pack_kernel(const float4* __restrict__ rec4, const T* __re
 // takes its whole jump.  It lies 2 nm + 0.005 % of r inside the sphere (the
 // fraction of the sphere itself is then at least the jump, by far more than
 // the rounding of the reference's arithmetic) and as far, and 1 % of r more,
-// outside the (r + tol) ball of every sphere of a lower structure that such
-// a walker's list can hold (none of them contains it or stops it).  The walk
-// uses them in iterations that stay within the near margin of the walker's
-// cell, so a point where a lower sphere meets this one lies within that
-// margin of the box, and both spheres are in the full list (membership
-// margin larger than the near one) of the cell the point falls or is clamped
-// to: the lists of the cells that the sphere's box covers hold them all.  A
-// warp per record; the squared radius is stored, -1 for none.
+// outside the (r + tol) ball of every sphere of a lower structure (none of
+// them contains the walker or stops it).  The walk uses them in iterations
+// that stay within the near margin of the walker's cell, so a point where a
+// lower sphere meets this one lies within that margin of the box, and the
+// near list of the cell that the point falls in or is clamped to holds the
+// lower sphere: the lists of the cells that this sphere meets hold them all.
+// A warp per record; the squared radius is stored, -1 for none.  80,000
+// records on 0.67 um cells take 0.37 ms, 0.56 ms over the full lists of every
+// cell of the sphere's box.
 template <typename T>
-__global__ void cells_safe_kernel(const float4* __restrict__ rec4, const int* __restrict__ rec_sid, int S,
-                                  const T* __restrict__ idx, const int* __restrict__ start,
-                                  const int* __restrict__ count, Grid g, float* __restrict__ safe) {
+__global__ void __launch_bounds__(256) cells_safe_kernel(const float4* __restrict__ rec4,
+                                                         const int* __restrict__ rec_sid, int S,
+                                                         const T* __restrict__ idx, const int* __restrict__ start,
+                                                         const int* __restrict__ count, Grid g,
+                                                         float* __restrict__ safe) {
   const int k = int((blockIdx.x * size_t(blockDim.x) + threadIdx.x) >> 5), lane = threadIdx.x & 31;
   if (k >= S) return;
   const float4 c = __ldg(rec4 + k);
   const int sid = __ldg(rec_sid + k);
   float best = c.w * 0.99995f - 2e-3f;
-  const float reach = c.w + 0.01f;
+  const float reach = c.w * 1.001f + 0.01f;
   const int nx = int(g.nLx), ny = int(g.nLy);
-  const int x0 = int(fminf(g.nLx - 1, fmaxf(0.f, floorf((c.x - reach + g.Lx / 2) / g.dLx))));
-  const int x1 = int(fminf(g.nLx - 1, fmaxf(0.f, floorf((c.x + reach + g.Lx / 2) / g.dLx))));
-  const int y0 = int(fminf(g.nLy - 1, fmaxf(0.f, floorf((c.y - reach + g.Ly / 2) / g.dLy))));
-  const int y1 = int(fminf(g.nLy - 1, fmaxf(0.f, floorf((c.y + reach + g.Ly / 2) / g.dLy))));
-  const int z0 = int(fminf(g.nLz - 1, fmaxf(0.f, floorf((c.z - reach + g.Lz / 2) / g.dLz))));
-  const int z1 = int(fminf(g.nLz - 1, fmaxf(0.f, floorf((c.z + reach + g.Lz / 2) / g.dLz))));
+  auto cell = [](float x, float L, float d, float n) {
+    return int(fminf(n - 1, fmaxf(0.f, floorf((x + L / 2) / d))));
+  };
+  const int x0 = cell(c.x - reach, g.Lx, g.dLx, g.nLx), x1 = cell(c.x + reach, g.Lx, g.dLx, g.nLx);
+  const int y0 = cell(c.y - reach, g.Ly, g.dLy, g.nLy), y1 = cell(c.y + reach, g.Ly, g.dLy, g.nLy);
+  const int z0 = cell(c.z - reach, g.Lz, g.dLz, g.nLz), z1 = cell(c.z + reach, g.Lz, g.dLz, g.nLz);
+  // distance of the centre from cell n of an axis; a boundary cell stands for
+  // all beyond it
+  auto gap = [](float x, int n, float L, float d, int last) {
+    const float lo = n == 0 ? -1e30f : n * d - L / 2, hi = n == last ? 1e30f : (n + 1) * d - L / 2;
+    return fmaxf(0.f, fmaxf(lo - x, x - hi));
+  };
   for (int p = z0; p <= z1; ++p)
-    for (int m = y0; m <= y1; ++m)
+    for (int m = y0; m <= y1; ++m) {
+      const float ez = gap(c.z, p, g.Lz, g.dLz, int(g.nLz) - 1), ey = gap(c.y, m, g.Ly, g.dLy, ny - 1);
       for (int n = x0; n <= x1; ++n) {
-        const int cell = (p * ny + m) * nx + n;
-        const int s = start[cell], e = s + count[cell];
+        const float ex = gap(c.x, n, g.Lx, g.dLx, nx - 1);
+        if (ex * ex + ey * ey + ez * ez > reach * reach) continue;
+        const int q = (p * ny + m) * nx + n;
+        const int s = start[q], e = s + count[q];
         for (int i = s + lane; i < e; i += 32) {
           const int o = int(idx[i]);
-          if (o >= S || __ldg(rec_sid + o) >= sid) continue;
+          if (o >= k || __ldg(rec_sid + o) >= sid) continue;  // records are in order of structures
           const float4 d = __ldg(rec4 + o);
-          const float ex = d.x - c.x, ey = d.y - c.y, ez = d.z - c.z;
-          const float gap = sqrtf(ex * ex + ey * ey + ez * ez) * 0.99999f - d.w * 1.00005f;
-          best = fminf(best, gap - 2e-3f - kTol - 0.01f * c.w);
+          const float fx = d.x - c.x, fy = d.y - c.y, fz = d.z - c.z;
+          const float apart = sqrtf(fx * fx + fy * fy + fz * fz) * 0.99999f - d.w * 1.00005f;
+          best = fminf(best, apart - 2e-3f - kTol - 0.01f * c.w);
         }
       }
+    }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) best = fminf(best, __shfl_xor_sync(0xffffffffu, best, o));
   if (lane == 0) safe[k] = best > 0.0f ? best * best : -1.0f;
@@ -1100,14 +1111,13 @@ extern "C" size_t nz_cells_pack_bytes(int n_items, int ncell, int S) {
 }
 
 extern "C" int nz_cells_pack(const float* rec4, const int* rec_sid, int S, const void* idx, int idx_bytes,
-                             const int* start, const int* count, int n_items, const void* full_idx,
-                             const int* full_start, const int* full_count, const nz_grid* grid, float margin,
+                             const int* start, const int* count, int n_items, const nz_grid* grid, float margin,
                              void* pack, void* stream) {
   int rc = check_grid(grid, "nz_cells_pack");
   if (rc) return rc;
   if (S < 0 || n_items < 0 || (idx_bytes != 2 && idx_bytes != 4) || !(margin > 0.0f) || !pack ||
-      (reinterpret_cast<uintptr_t>(pack) & 15) || !start || !count || !full_start || !full_count ||
-      (S > 0 && (!rec4 || !rec_sid || !full_idx)) || (n_items > 0 && !idx) ||
+      (reinterpret_cast<uintptr_t>(pack) & 15) || !start || !count || (S > 0 && (!rec4 || !rec_sid)) ||
+      (n_items > 0 && !idx) ||
       (reinterpret_cast<uintptr_t>(rec4) & 15))
     return set_error(NZ_ERR_ARG, "nz_cells_pack: bad arguments (S=%d items=%d idx_bytes=%d)", S, n_items, idx_bytes);
   if (!(grid->dLx <= 1e4f && grid->dLy <= 1e4f && grid->dLz <= 1e4f))
@@ -1116,26 +1126,22 @@ extern "C" int nz_cells_pack(const float* rec4, const int* rec_sid, int S, const
   if (ncell + n_items > 0x7fffffffll) return set_error(NZ_ERR_ARG, "nz_cells_pack: too many cells and entries");
   const Grid g{grid->Lx, grid->Ly, grid->Lz, grid->dLx, grid->dLy, grid->dLz, float(grid->nx), float(grid->ny),
                float(grid->nz)};
-  const double h = 0.5 * sqrt(double(g.dLx) * g.dLx + double(g.dLy) * g.dLy + double(g.dLz) * g.dLz);
+  const float h = float(0.5 * sqrt(double(g.dLx) * g.dLx + double(g.dLy) * g.dLy + double(g.dLz) * g.dLz));
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const unsigned blocks = unsigned((ncell + 127) / 128);
+  const unsigned blocks = unsigned((8 * ncell + 255) / 256);
   const float4* r = reinterpret_cast<const float4*>(rec4);
   uint4* out = static_cast<uint4*>(pack);
   float* safe = reinterpret_cast<float*>(out + pack_pairs(n_items, int(ncell)));
   const unsigned sblocks = unsigned((size_t(S) * 32 + 255) / 256);
   if (idx_bytes == 2)
-    cells_pack_kernel<<<blocks, 128, 0, st>>>(r, static_cast<const uint16_t*>(idx), start, count, g, h,
-                                              double(margin), out);
+    cells_pack_kernel<<<blocks, 256, 0, st>>>(r, static_cast<const uint16_t*>(idx), start, count, g, h, margin, out);
   else
-    cells_pack_kernel<<<blocks, 128, 0, st>>>(r, static_cast<const int*>(idx), start, count, g, h, double(margin),
-                                              out);
+    cells_pack_kernel<<<blocks, 256, 0, st>>>(r, static_cast<const int*>(idx), start, count, g, h, margin, out);
   rc = check_launch("cells_pack_kernel");
   if (rc || S == 0) return rc;
   if (idx_bytes == 2)
-    cells_safe_kernel<<<sblocks, 256, 0, st>>>(r, rec_sid, S, static_cast<const uint16_t*>(full_idx), full_start,
-                                               full_count, g, safe);
+    cells_safe_kernel<<<sblocks, 256, 0, st>>>(r, rec_sid, S, static_cast<const uint16_t*>(idx), start, count, g, safe);
   else
-    cells_safe_kernel<<<sblocks, 256, 0, st>>>(r, rec_sid, S, static_cast<const int*>(full_idx), full_start,
-                                               full_count, g, safe);
+    cells_safe_kernel<<<sblocks, 256, 0, st>>>(r, rec_sid, S, static_cast<const int*>(idx), start, count, g, safe);
   return check_launch("cells_safe_kernel");
 }

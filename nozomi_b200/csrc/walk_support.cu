@@ -12,6 +12,7 @@ namespace nz {
 // kernel and bounded.  The label of a point is found from its cell's list:
 // every sphere that contains a point of a cell is a member of that cell.
 // ---------------------------------------------------------------------------
+template <int LK>
 __global__ void seed_kernel(nz_substrate sub, const uint8_t* __restrict__ target, uint32_t id0, int N, uint32_t k0,
                             uint32_t k1, uint32_t stream, int max_rounds, float* __restrict__ spins,
                             int* __restrict__ label, int* __restrict__ n_unseeded) {
@@ -33,7 +34,19 @@ __global__ void seed_kernel(nz_substrate sub, const uint8_t* __restrict__ target
     const int cell = cell_of(g, px, py, pz);
     const int start = sub.cell_start[cell], count = sub.cell_count[cell];
     int lab = ns;
-    for (int n = 0; n < count; ++n) {
+    if constexpr (LK != 0) {  // index lists: structures ascend, the first containing entry decides
+      for (int n = 0; n < count; ++n) {
+        const int key = LK == 2 ? int(static_cast<const unsigned short*>(sub.cell_idx)[start + n])
+                                : static_cast<const int*>(sub.cell_idx)[start + n];
+        const float4 c = __ldg(reinterpret_cast<const float4*>(sub.rec4) + key);
+        const float dx = px - c.x, dy = py - c.y, dz = pz - c.z;
+        if (dx * dx + dy * dy + dz * dz - c.w * c.w < 0) {
+          lab = sub.rec_sid[key];
+          break;
+        }
+      }
+    }
+    for (int n = 0; LK == 0 && n < count; ++n) {
       const int s = sub.cell_items[start + n];
       const float dx = px - cx[s], dy = py - cx[S + s], dz = pz - cx[2 * S + s];
       const int sid = int(sphSID[s]);
@@ -332,8 +345,22 @@ extern "C" int nz_seed_range(const nz_substrate* sub, const uint8_t* target, uin
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (cudaMemsetAsync(n_unseeded, 0, sizeof(int), st) != cudaSuccess) return check_launch("nz_seed memset");
   if (N == 0) return NZ_OK;
-  seed_kernel<<<(N + 255) / 256, 256, 0, st>>>(*sub, target, id0, N, key0, key1, stream_id, max_rounds, spins,
-                                                label, n_unseeded);
+  // index lists, where the substrate has them: a record an entry instead of
+  // five arrays, and no entry past the first that contains the point (2e5
+  // walkers in axons on 20^3 cells: 0.33 ms against 0.45)
+  const int width = sub->cell_idx && sub->rec4 && sub->rec_sid && (reinterpret_cast<uintptr_t>(sub->rec4) & 15) == 0
+                        ? sub->idx_bytes & ~NZ_NEAR_PACKED
+                        : 0;
+  const unsigned blocks = unsigned((N + 255) / 256);
+  if (width == 2 && sub->S <= 65536)
+    seed_kernel<2><<<blocks, 256, 0, st>>>(*sub, target, id0, N, key0, key1, stream_id, max_rounds, spins, label,
+                                           n_unseeded);
+  else if (width == 4)
+    seed_kernel<4><<<blocks, 256, 0, st>>>(*sub, target, id0, N, key0, key1, stream_id, max_rounds, spins, label,
+                                           n_unseeded);
+  else
+    seed_kernel<0><<<blocks, 256, 0, st>>>(*sub, target, id0, N, key0, key1, stream_id, max_rounds, spins, label,
+                                           n_unseeded);
   return check_launch("seed_kernel");
 }
 

@@ -173,8 +173,8 @@ class DeviceSubstrate:
         lib = L.load()
         pack = torch.empty(int(lib.nz_cells_pack_bytes(n, self.ncell, self.S)), dtype=torch.uint8, device=_dev())
         L.check(lib.nz_cells_pack(_p(self.rec4), _p(self.rec_sid), self.S, _p(idx), self.idx_bytes, _p(start),
-                                  _p(count), n, _p(self.cell_idx), _p(self.cell_start), _p(self.cell_count),
-                                  L.byref(self.grid), np.float32(margin), _p(pack), _stream()), "nz_cells_pack")
+                                  _p(count), n, L.byref(self.grid), np.float32(margin), _p(pack), _stream()),
+                "nz_cells_pack")
         return pack
 
     def _build_cells(self, margin: float | None = None, store: bool = True, rounded: bool = False):
