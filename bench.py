@@ -80,21 +80,21 @@ KERNEL_SOURCES = ("nozomi_b200/csrc/walk_fused.cu", "nozomi_b200/csrc/nz_common.
 # dram__bytes_write.sum) of the captured launch, divided by the walker-steps
 # that launch ran; kernel_sha: the sources' hash at capture.
 PROFILED = {
-    "packed": {"kernel_sha": "142940ca4a9a2176", "warp_inst_per_walker_step": 40.982,
-               "dram_bytes_per_walker_step": 1.7926,
+    "packed": {"kernel_sha": "61c30e018a04ea72", "warp_inst_per_walker_step": 40.989,
+               "dram_bytes_per_walker_step": 1.7954,
                "shape": {"cell": 0.5, "near_margin": 0.5, "coarsen": 8, "threads": 128, "lists": "index",
                          "near_shape": "round", "stage": 0},
                "capture": "walk_fused_kernel<PHI, idx16> launch 3 of `python bench.py --workload packed --walkers "
                           "1000000 --steps-per-launch 200 --steps 1 --warmup 1 --no-cpu-baseline --e2e-steps 0` "
-                          "(200,000,000 walker-steps): 8,196,434,206 warp instructions, 358.5 MB DRAM"},
-    "batched": {"kernel_sha": "142940ca4a9a2176", "warp_inst_per_walker_step": 32.992,
-                "dram_bytes_per_walker_step": 0.5633,
+                          "(200,000,000 walker-steps): 8,197,826,067 warp instructions, 359.1 MB DRAM"},
+    "batched": {"kernel_sha": "61c30e018a04ea72", "warp_inst_per_walker_step": 32.993,
+                "dram_bytes_per_walker_step": 0.5656,
                 "shape": {"cell": 1.0, "near_margin": 0.5, "coarsen": 4, "threads": 256, "lists": "index",
                           "near_shape": "round", "stage": 0},
                 "capture": "walk_fused_kernel<PHI, idx16> launch 2 of `python bench.py --walker-scale 0.1 --steps 1 "
                            "--warmup 1 --no-serving --no-plain --no-cpu-baseline --e2e-steps 0 --no-autotune --cell 1.0 "
                            "--coarsen 4 --steps-per-launch 2000 --threads 256` (64 jobs, 2,407,477,000 walker-steps): "
-                           "79,428,198,810 warp instructions, 1356.2 MB DRAM"},
+                           "79,429,692,403 warp instructions, 1361.8 MB DRAM"},
 }
 
 
