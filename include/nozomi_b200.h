@@ -244,7 +244,7 @@ int nz_cells_index(const int* items, int n_items, const int* perm, int S, const 
  * record's centre meets no sphere.  idx, start, count: the near lists, laid
  * out without gaps (start the exclusive scan of count).  pack: nz_cells_pack_bytes(n_items, ncell, S) bytes, 16-byte
  * aligned; nz_substrate.near_items must then be n_items.  Grids with a cell
- * edge above 1e4 um are refused. */
+ * edge above 1e4 um and margins above 100 um are refused. */
 size_t nz_cells_pack_bytes(int n_items, int ncell, int S);
 int nz_cells_pack(const float* rec4, const int* rec_sid, int S, const void* idx, int idx_bytes, const int* start,
                   const int* count, int n_items, const nz_grid* grid, float margin, void* pack, void* stream);

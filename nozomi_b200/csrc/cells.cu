@@ -705,7 +705,10 @@ __global__ void index_fill_kernel(const int* __restrict__ items, int n, const in
 //   of R + 2 % reach and its square                     2 u rho
 // E is their sum and 15 % more (10 nm for r = 1 um, 0.5 um cells and margin).
 // Spheres that half precision holds badly (R above 100 um, centres beyond
-// 200 um) get R = inf: always near.
+// 200 um) get R = inf: always near.  M is at most 100 um (kPackMargin), so a
+// sphere in reach is within 200 um and d^2 below the largest half (255.9^2).
+constexpr float kPackMargin = 100.0f;
+
 __device__ __forceinline__ void pack_entry(float4 c, float ox, float oy, float oz, float h, float M, __half* v) {
   const float x = c.x - ox, y = c.y - oy, z = c.z - oz;  // single precision: its rounding is in the 15 %
   const float u = 1.0f / 2048, rho = c.w + kTol, m = h + 2 * M + rho;
@@ -1122,6 +1125,7 @@ extern "C" int nz_cells_pack(const float* rec4, const int* rec_sid, int S, const
     return set_error(NZ_ERR_ARG, "nz_cells_pack: bad arguments (S=%d items=%d idx_bytes=%d)", S, n_items, idx_bytes);
   if (!(grid->dLx <= 1e4f && grid->dLy <= 1e4f && grid->dLz <= 1e4f))
     return set_error(NZ_ERR_ARG, "nz_cells_pack: cell edges above 1e4 um");
+  if (!(margin <= kPackMargin)) return set_error(NZ_ERR_ARG, "nz_cells_pack: margin above 100 um");
   const long long ncell = 1ll * grid->nx * grid->ny * grid->nz;
   if (ncell + n_items > 0x7fffffffll) return set_error(NZ_ERR_ARG, "nz_cells_pack: too many cells and entries");
   const Grid g{grid->Lx, grid->Ly, grid->Lz, grid->dLx, grid->dLy, grid->dLz, float(grid->nx), float(grid->ny),

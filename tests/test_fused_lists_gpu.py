@@ -94,3 +94,20 @@ def test_walkers_spread_over_warps(N):
     sub = engine.DeviceSubstrate(*args, near_margin=0.5)
     x, _ = engine.seed(sub, range(ns + 1), N, key=4)
     _same(_fused(sub, x, 9, 12), _plain(engine.DeviceSubstrate(*args, idx_bytes=0), x, 9, 12))
+
+
+# jumps and margins of hundreds of um: squared distances of spheres within
+# reach pass the largest half-precision number
+@pytest.mark.parametrize("margin,D", [(90.0, 3e4), (300.0, 1e6)])
+def test_long_jumps_match_the_array_step(margin, D):
+    from nozomi_b200 import engine
+    rng = np.random.default_rng(11)
+    S, L, N, ns = 60, (1500.0, 1500.0, 1500.0), 4000, 4
+    sph = np.zeros((5, S))
+    sph[:3] = rng.uniform(-700.0, 700.0, (3, S))
+    sph[3] = rng.uniform(60.0, 98.0, S)
+    sph[4] = rng.integers(0, ns, S)
+    x = torch.from_numpy(rng.uniform(-750.0, 750.0, (3, N)).astype(np.float32)).cuda()
+    args = (sph, ns, L, (3, 3, 3), np.full(ns + 1, D), np.full(ns + 1, 80.0))
+    want = _plain(engine.DeviceSubstrate(*args, jump_tol=700.0, idx_bytes=0), x, 5)
+    _same(_fused(engine.DeviceSubstrate(*args, jump_tol=700.0, near_margin=margin), x, 5), want)
