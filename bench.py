@@ -80,21 +80,21 @@ KERNEL_SOURCES = ("nozomi_b200/csrc/walk_fused.cu", "nozomi_b200/csrc/nz_common.
 # dram__bytes_write.sum) of the captured launch, divided by the walker-steps
 # that launch ran; kernel_sha: the sources' hash at capture.
 PROFILED = {
-    "packed": {"kernel_sha": "db1cf1fe48e3dbca", "warp_inst_per_walker_step": 40.992,
-               "dram_bytes_per_walker_step": 1.8069,
+    "packed": {"kernel_sha": "aa15194f838fa36b", "warp_inst_per_walker_step": 40.990,
+               "dram_bytes_per_walker_step": 1.8011,
                "shape": {"cell": 0.5, "near_margin": 0.5, "coarsen": 8, "threads": 128, "lists": "index",
                          "near_shape": "round", "stage": 0},
                "capture": "walk_fused_kernel<PHI, idx16> launch 3 of `python bench.py --workload packed --walkers "
                           "1000000 --steps-per-launch 200 --steps 1 --warmup 1 --no-cpu-baseline --e2e-steps 0` "
-                          "(200,000,000 walker-steps): 8,198,445,927 warp instructions, 361.4 MB DRAM"},
-    "batched": {"kernel_sha": "db1cf1fe48e3dbca", "warp_inst_per_walker_step": 32.994,
-                "dram_bytes_per_walker_step": 0.5632,
+                          "(200,000,000 walker-steps): 8,198,067,851 warp instructions, 360.2 MB DRAM"},
+    "batched": {"kernel_sha": "aa15194f838fa36b", "warp_inst_per_walker_step": 32.993,
+                "dram_bytes_per_walker_step": 0.5611,
                 "shape": {"cell": 1.0, "near_margin": 0.5, "coarsen": 4, "threads": 256, "lists": "index",
                           "near_shape": "round", "stage": 0},
                 "capture": "walk_fused_kernel<PHI, idx16> launch 2 of `python bench.py --walker-scale 0.1 --steps 1 "
                            "--warmup 1 --no-serving --no-plain --no-cpu-baseline --e2e-steps 0 --no-autotune --cell 1.0 "
                            "--coarsen 4 --steps-per-launch 2000 --threads 256` (64 jobs, 2,407,477,000 walker-steps): "
-                           "79,431,172,024 warp instructions, 1355.9 MB DRAM"},
+                           "79,430,203,761 warp instructions, 1350.7 MB DRAM"},
 }
 
 

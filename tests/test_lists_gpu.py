@@ -1,6 +1,8 @@
 """The padded cell table at the sizes where its selection can go wrong,
 against the oracle's table (same distances, same order of ties), which is
 pinned to the reference's."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -88,3 +90,21 @@ def test_member_near_and_index_lists(S, L, nseg, order):
             mem = members[cs[c]:cs[c] + cc[c]]
             assert (np.diff(mem) > 0).all()
             np.testing.assert_array_equal(idx[cs[c]:cs[c] + cc[c]], np.sort(perm[mem]))
+
+
+# out of place, in place, and out one element before in
+@pytest.mark.parametrize("shift", [None, 0, 1])
+@pytest.mark.parametrize("n", [1, 9000, 100_003])
+def test_scan_in_place_and_overlapping(n, shift):
+    from nozomi_b200 import _lib as L
+    v = np.random.default_rng(n).integers(0, 9, n).astype(np.int32)
+    buf = torch.zeros(n + 1, dtype=torch.int32, device="cuda")
+    src = buf[(shift or 0):][:n]
+    src.copy_(torch.from_numpy(v))
+    out = torch.empty(n, dtype=torch.int32, device="cuda") if shift is None else buf[:n]
+    total = torch.zeros(1, dtype=torch.int32, device="cuda")
+    L.check(L.load().nz_exclusive_scan_i32(ctypes.c_void_p(src.data_ptr()), ctypes.c_void_p(out.data_ptr()), n,
+                                           ctypes.c_void_p(total.data_ptr()), None), "nz_exclusive_scan_i32")
+    torch.cuda.synchronize()
+    np.testing.assert_array_equal(out.cpu().numpy(), np.cumsum(v) - v)
+    assert int(total.item()) == v.sum()
