@@ -209,7 +209,7 @@ __global__ void __launch_bounds__(kSigMaxThreads) signal_kernel(nz_state st, con
                                                                 int groups, int per_block, double* __restrict__ out) {
   __shared__ float4 s_p[kSigTile];
   __shared__ double s_sum[2][kSigMaxThreads];
-  const int t = threadIdx.x, group = t / combos, combo = blockIdx.y * combos + t % combos;
+  const int t = threadIdx.x, group = t / combos, combo = blockIdx.x * combos + t % combos;
   const bool busy = group < groups && combo < ndir * nb;
   float d0 = 0.f, d1 = 0.f, d2 = 0.f, a0 = 0.f;
   if (busy) {
@@ -220,7 +220,7 @@ __global__ void __launch_bounds__(kSigMaxThreads) signal_kernel(nz_state st, con
     a0 = amp[combo % nb];
   }
   double re = 0.0, im = 0.0;
-  const int first = blockIdx.x * per_block, last = min(st.N, first + per_block);
+  const int first = blockIdx.y * per_block, last = min(st.N, first + per_block);
   for (int base = first; base < last; base += kSigTile) {
     const int n = min(kSigTile, last - base);
     __syncthreads();
@@ -486,10 +486,10 @@ extern "C" int nz_signal_phi(const nz_state* st, const float* dirs, int ndir, co
     }
   }
   // one wave of blocks (32 registers a thread: full SMs), each at least 64
-  // walkers
+  // walkers (at most 148 * 64 of them, the grid's y)
   const int wave = std::max(1, 148 * (2048 / threads) / ny);
   const int per_block = std::max(64, (st->N + wave - 1) / wave);
-  signal_kernel<<<dim3(unsigned((st->N + per_block - 1) / per_block), unsigned(ny)), threads, 0,
+  signal_kernel<<<dim3(unsigned(ny), unsigned((st->N + per_block - 1) / per_block)), threads, 0,
                   static_cast<cudaStream_t>(stream)>>>(*st, dirs, ndir, amp, nb, combos, groups, per_block, out);
   return check_launch("signal_kernel");
 }

@@ -71,3 +71,23 @@ def test_a_walker_adds_the_same_numbers_wherever_it_stands():
         np.testing.assert_array_equal(sums([v, 0.0]) - zero, alone)
         np.testing.assert_array_equal(sums([0.0, 0.0, v]) - 2 * zero, alone)
         np.testing.assert_allclose(sums([v, 3.0e5]) - big, alone, rtol=0, atol=1e-15)
+
+
+def test_signal_of_many_pairs():
+    """More (direction, b) pairs than 65,535 blocks hold; the last and a few
+    others against 64 bits, with the bound above."""
+    from nozomi_b200 import engine
+    ndir, nb, N = 70_000, 370, 3
+    rng = np.random.default_rng(1)
+    phi = np.zeros((6, N), np.float32)
+    phi[:3] = rng.normal(0, 1.0, (3, N))
+    d = rng.standard_normal((3, ndir)).astype(np.float32)
+    amps = np.linspace(0.0, 2.5, nb).astype(np.float32)
+    x = torch.zeros((3, N), device="cuda")
+    st = engine.FusedState.from_walkers(engine.Walkers(x, x.clone(), phi=torch.from_numpy(phi).cuda()))
+    out = st.signal(torch.from_numpy(d).cuda().contiguous(), torch.from_numpy(amps).cuda())
+    for i in (0, 1, 33_333, ndir - 1):
+        ph = (phi[0] * d[0, i] + phi[1] * d[1, i]) + phi[2] * d[2, i]
+        a = (amps[:, None] * ph[None]).astype(np.float64)
+        want = np.stack([np.cos(a).sum(1), np.sin(a).sum(1)])
+        assert np.abs(out[:, i].cpu().numpy() - want).max() <= N * 2.0**-22
