@@ -377,7 +377,7 @@ __device__ __forceinline__ int step_cell(const JobDev& J, float x, float y, floa
   mx = __fmaf_rn(cx, g.dLx, 0.5f * (g.dLx - g.Lx));
   my = __fmaf_rn(cy, g.dLy, 0.5f * (g.dLy - g.Ly));
   mz = __fmaf_rn(cz, g.dLz, 0.5f * (g.dLz - g.Lz));
-  return int(cz * g.nLx * g.nLy + cy * g.nLx + cx);
+  return cell_index(g, cx, cy, cz);
 }
 
 // Start and count of cell `cell`'s list (the near list when near).  In the
