@@ -96,14 +96,32 @@ __device__ __forceinline__ void entry(const void* __restrict__ list, const float
   }
 }
 
+// This iteration's reach |j| * jump_remaining, from the hardware reciprocal
+// square root: within a few ulp of sqrtf, far inside the 2 % + 2 nm of slack
+// of the only two uses (the near test and the first-pass filter), which
+// decide what is scanned, never a result.
+__device__ __forceinline__ float reach_of(float a, float jr) { return a * rsqrtf(fmaxf(a, 1e-30f)) * jr; }
+
+// Jumps below this squared length (1e-4 um; none at all where D is 0) are too
+// short for the filters' arithmetic, which mark every entry then.  beyond
+// passes over the spheres that the segment cannot come near, with the filter
+// of scan_cell: with no jump at all the quadratic has no roots, and the
+// fraction of an outside sphere would be 0 at any distance.
+constexpr float kTinyJump2 = 1e-8f;
+__device__ __forceinline__ bool beyond(float dx, float dy, float dz, float r, float a, float jr) {
+  if (a >= kTinyJump2) return false;
+  const float ro = r + (kTol + reach_of(a, jr) * 1.02f + 2e-3f);
+  return !(__fmaf_rn(dx, dx, __fmaf_rn(dy, dy, dz * dz)) <= ro * ro);
+}
+
 // The reference's collision pass over one cell's list for one walker of
 // known label (sim3d_kernel.cu:800-830), lane by lane: only for the rare
 // iteration whose label had to be corrected.
 template <int LK, bool T64, bool SH>
 __device__ __noinline__ void scan_lane(const void* __restrict__ list, const float4* __restrict__ rec,
                                           const int* __restrict__ sid, int start, int count, int lo, int hi, float x,
-                                          float y, float z, float a, float jx, float jy, float jz, int S, int& oob,
-                                          ScanOut& o) {
+                                          float y, float z, float a, float jx, float jy, float jz, float jr, int S,
+                                          int& oob, ScanOut& o) {
   o.fin = 0.0f;
   o.fout = kBig;
   o.any_in = false;
@@ -113,6 +131,7 @@ __device__ __noinline__ void scan_lane(const void* __restrict__ list, const floa
     entry<LK, SH>(list, rec, sid, start + i, S, oob, key, c);
     if (key >= hi) break;
     const float dx = x - c.x, dy = y - c.y, dz = z - c.z;
+    if (beyond(dx, dy, dz, c.w, a, jr)) continue;
     const bool inside = dx * dx + dy * dy + dz * dz - c.w * c.w < 0;
     if (inside || key < lo) {
       const float f = step_either_t<T64>(inside, dx, dy, dz, c.w, a, jx, jy, jz);
@@ -216,7 +235,8 @@ template <int LK, bool T64, bool SH>
 __device__ __forceinline__ void fractions(uint32_t bits, const void* __restrict__ list,
                                           const float4* __restrict__ rec, const int* __restrict__ sid, int first,
                                           int lo, int hi, float x, float y, float z, float a, float jx, float jy,
-                                          float jz, int S, int& oob, ScanOut& o, bool& lower, int& within) {
+                                          float jz, float jr, int S, int& oob, ScanOut& o, bool& lower,
+                                          int& within) {
   while (bits) {
     const int i = bit_entry(__ffs(bits) - 1);
     bits &= bits - 1u;
@@ -226,6 +246,7 @@ __device__ __forceinline__ void fractions(uint32_t bits, const void* __restrict_
     if (key >= hi) continue;
     const bool below = key < lo;
     const float dx = x - c.x, dy = y - c.y, dz = z - c.z;
+    if (beyond(dx, dy, dz, c.w, a, jr)) continue;
     const float d2 = dx * dx + dy * dy + dz * dz;
     const bool inside = d2 - c.w * c.w < 0;
     if (inside || below) {
@@ -400,12 +421,6 @@ __device__ __forceinline__ void cell_list(const JobDev& J, bool near, int cell, 
   }
 }
 
-// This iteration's reach |j| * jump_remaining, from the hardware reciprocal
-// square root: within a few ulp of sqrtf, far inside the 2 % + 2 nm of slack
-// of the only two uses (the near test and the first-pass filter), which
-// decide what is scanned, never a result.
-__device__ __forceinline__ float reach_of(float a, float jr) { return a * rsqrtf(fmaxf(a, 1e-30f)) * jr; }
-
 // Draw `draw` of step s scaled by ds.
 __device__ __forceinline__ void jump_of(const JobDev& J, uint32_t wid, int s, int draw, float ds, float& jx, float& jy,
                                         float& jz) {
@@ -509,7 +524,7 @@ __device__ __forceinline__ void walk_warp(const JobDev& J, bool live, int w, int
     // sphere that held the walker longest when its fractions were last
     // computed.
     bool deep = false;
-    if (LK != 0 && J.rec_safe && within >= lo && within < hi && near && a >= 1e-8f) {
+    if (LK != 0 && J.rec_safe && within >= lo && within < hi && near && a >= kTinyJump2) {
       const float4 c = SH ? s_stage[within] : __ldg(J.rec4 + within);
       const float safe = __ldg(J.rec_safe + within);
       const float dx = x - c.x, dy = y - c.y, dz = z - c.z;
@@ -530,7 +545,7 @@ __device__ __forceinline__ void walk_warp(const JobDev& J, bool live, int w, int
     bool lower = false;
     bool more = act && !deep && count > 0;
     const bool packed = LK != 0 && J.near_pack != nullptr;
-    const bool tiny = a < 1e-8f;  // a jump too short for the filter's arithmetic: every entry is near
+    const bool tiny = a < kTinyJump2;  // every entry is marked; fractions passes over the far ones
     const float inf = __int_as_float(0x7f800000);
     const void* list = LK ? (near ? J.near_idx : J.idx) : nullptr;
     const float4* rec = LK ? J.rec4 : (near ? J.near_sph4 : J.sph4);
@@ -601,8 +616,8 @@ __device__ __forceinline__ void walk_warp(const JobDev& J, bool live, int w, int
         }
       }
       if (bits)
-        fractions<LK, kT64, SH>(bits, list, rec, sid, start + base, lo, hi, x, y, z, a, jx, jy, jz, J.S, oob, r, lower,
-                                within);
+        fractions<LK, kT64, SH>(bits, list, rec, sid, start + base, lo, hi, x, y, z, a, jx, jy, jz, jr, J.S, oob, r,
+                                lower, within);
       more = more && base + 32 < count;
     }
     if (!act) continue;
@@ -630,7 +645,7 @@ __device__ __forceinline__ void walk_warp(const JobDev& J, bool live, int w, int
       int fs, fc;
       cell_list(J, false, cell, fs, fc, oob);
       scan_lane<LK, kT64, SH>(LK ? J.idx : nullptr, LK ? J.rec4 : J.sph4, LK ? nullptr : J.sid, fs, fc, lo, hi, x, y,
-                              z, a, jx, jy, jz, J.S, oob, r);
+                              z, a, jx, jy, jz, jr, J.S, oob, r);
     }
     jc = ref_min(jc, r.any_in ? r.fin : kBig);
     jc = ref_min(jc, r.fout);
