@@ -51,7 +51,7 @@ def test_more_than_2_24_cells():
     args = (sph, ns, L)
     D = (np.full(ns + 1, 2.0), np.full(ns + 1, 80.0))
     want = _walk(engine.DeviceSubstrate(*args, (24, 24, 24), *D, idx_bytes=0), x, 8)
-    assert (want.label.cpu().numpy() < ns).mean() > 0.3  # half in spheres, half among them
+    assert 0.2 < (want.label.cpu().numpy() < ns).mean() < 0.8  # walkers in the spheres and among them
     spins, label = engine.seed(engine.DeviceSubstrate(*args, (24, 24, 24), *D), range(ns), 500, key=3)
     for idx in (2, 4, 0):
         sub = engine.DeviceSubstrate(*args, (300, 300, 300), *D, near_margin=0.6, idx_bytes=idx)
