@@ -269,8 +269,8 @@ int sort_lists(const int* start, const int* count, int ncell, int S, T* list, cu
   if (rc) return rc;
   size_t bytes = 0;
   if (S <= kBitmapKeys) bytes = size_t((S + 31) / 32) * sizeof(unsigned);
-  if (bytes > 48 * 1024 &&
-      cudaFuncSetAttribute(long_lists_sort_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  // at every size: the 48 KiB allowed without it are for static and dynamic bytes together
+  if (cudaFuncSetAttribute(long_lists_sort_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            kBitmapKeys / 8) != cudaSuccess)
     return check_launch("long_lists_sort_kernel attribute");
   const int ctas = (ncell + 255) / 256 < 148 * 4 ? (ncell + 255) / 256 : 148 * 4;
