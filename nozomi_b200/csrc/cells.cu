@@ -8,6 +8,7 @@
 // boundary distances of its bounding box are below jump_tol.  The predicate is
 // separable per axis and, per axis, monotone in the cell index, so each sphere
 // enumerates only the box of cells it can belong to.
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <cuda_fp16.h>
@@ -107,9 +108,12 @@ __global__ void __launch_bounds__(256) cells_members_kernel(const double* __rest
   }
 }
 
-// Ascending order within each cell's list, keys in [0, S).  A warp per cell
-// for lists of up to kWarpSort entries: nothing to do when they ascend
-// already, else a bitonic sort in registers, entry 32 k + lane in v[k].
+// Ascending order within each cell's list, keys in [0, S).  A warp per list of
+// up to kWarpSort entries: nothing to do when they ascend already, else a
+// bitonic sort in registers, entry 32 k + lane in v[k].  A CTA notes the
+// lists of two and more entries among its `chunk` cells (nearly all cells of a
+// fine grid in a nearly empty box have none: a warp launched for each of 8e6
+// cells took 0.53 ms) and its warps take them in turn.
 // Bound by its compare-exchanges (21 rounds for 33-64 entries).  One thread
 // per cell and a heapsort in memory took 2.1 ms for two lists of 420,000
 // cells (57 entries a cell in one of them), this
@@ -165,21 +169,30 @@ __device__ __forceinline__ void sort_list(T* a, int n, int lane) {
 
 template <typename T>
 __global__ void __launch_bounds__(256) lists_sort_kernel(const int* __restrict__ start, const int* __restrict__ count,
-                                                         int ncell, T* __restrict__ list) {
-  const int c = int((blockIdx.x * size_t(blockDim.x) + threadIdx.x) >> 5), lane = threadIdx.x & 31;
-  if (c >= ncell) return;
-  const int n = count[c];
-  if (n < 2 || n > kWarpSort) return;
-  T* a = list + start[c];
-  if (n <= 32) sort_list<1>(a, n, lane);
-  else if (n <= 64) sort_list<2>(a, n, lane);
-  else sort_list<4>(a, n, lane);
+                                                         int ncell, int chunk, T* __restrict__ list) {
+  __shared__ int s_cells[256], s_n;
+  const int t = threadIdx.x, lane = t & 31;
+  if (t == 0) s_n = 0;
+  __syncthreads();
+  const long long mine = 1ll * blockIdx.x * chunk + t;
+  if (t < chunk && mine < ncell && count[mine] >= 2 && count[mine] <= kWarpSort)
+    s_cells[atomicAdd(&s_n, 1)] = int(mine);
+  __syncthreads();
+  for (int q = t >> 5; q < s_n; q += 8) {
+    const int c = s_cells[q], n = count[c];
+    T* a = list + start[c];
+    if (n <= 32) sort_list<1>(a, n, lane);
+    else if (n <= 64) sort_list<2>(a, n, lane);
+    else sort_list<4>(a, n, lane);
+  }
 }
 
 // Longer lists (coarse grids): a CTA per list marks its entries in a bitmap
-// of the S keys in shared memory and reads them back in order.  CTAs look
-// over the cells 256 at a time.  Lists with repeats, or more keys than the
-// bitmap holds, are heapsorted by one thread.
+// of the S keys in shared memory and reads them back in order, unless they
+// ascend already.  CTAs look over `chunk` cells at a time, few enough that a
+// coarse grid's lists reach every SM.  Lists with repeats are heapsorted by
+// one thread; with more keys than the bitmap holds every thread heapsorts a
+// list.
 template <typename T>
 __device__ void heapsort(T* a, int n) {
   auto sift = [&](int root, int end) {
@@ -206,27 +219,36 @@ constexpr int kBitmapKeys = 1 << 20;  // 128 KiB of shared memory
 
 template <typename T>
 __global__ void __launch_bounds__(256) long_lists_sort_kernel(const int* __restrict__ start,
-                                                              const int* __restrict__ count, int ncell, int S,
-                                                              T* __restrict__ list) {
+                                                              const int* __restrict__ count, int ncell, int chunk,
+                                                              int S, T* __restrict__ list) {
   extern __shared__ unsigned s_bits[];  // (S + 31) / 32 words, or none beyond kBitmapKeys keys
   __shared__ int s_cells[256];
   __shared__ int s_n, s_repeats, s_before[8];
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const int words = (S + 31) / 32;
-  for (int base = blockIdx.x * 256; base < ncell; base += gridDim.x * 256) {
+  for (long long base = 1ll * blockIdx.x * chunk; base < ncell; base += 1ll * gridDim.x * chunk) {
+    const bool is_long = t < chunk && base + t < ncell && count[base + t] > kWarpSort;
+    if (S > kBitmapKeys) {
+      if (!is_long) continue;
+      T* a = list + start[base + t];
+      const int n = count[base + t];
+      int i = 1;
+      while (i < n && a[i - 1] <= a[i]) ++i;
+      if (i < n) heapsort(a, n);
+      continue;
+    }
     __syncthreads();
     if (t == 0) s_n = 0;
     __syncthreads();
-    if (base + t < ncell && count[base + t] > kWarpSort) s_cells[atomicAdd(&s_n, 1)] = base + t;
+    if (is_long) s_cells[atomicAdd(&s_n, 1)] = int(base) + t;
     __syncthreads();
     const int found = s_n;
     for (int q = 0; q < found; ++q) {
       const int c = s_cells[q], n = count[c];
       T* a = list + start[c];
-      if (S > kBitmapKeys) {
-        if (t == 0) heapsort(a, n);
-        continue;
-      }
+      bool sorted = true;
+      for (int i = t + 1; i < n; i += 256) sorted &= a[i - 1] <= a[i];
+      if (__syncthreads_and(sorted)) continue;
       for (int w = t; w < words; w += 256) s_bits[w] = 0u;
       if (t == 0) s_repeats = 0;
       __syncthreads();
@@ -264,7 +286,9 @@ __global__ void __launch_bounds__(256) long_lists_sort_kernel(const int* __restr
 // Both kernels over a set of lists with keys below S.
 template <typename T>
 int sort_lists(const int* start, const int* count, int ncell, int S, T* list, cudaStream_t st) {
-  lists_sort_kernel<T><<<unsigned((size_t(ncell) * 32 + 255) / 256), 256, 0, st>>>(start, count, ncell, list);
+  // cells of a CTA: a list a warp for few cells, four waves of CTAs (8 an SM) for more
+  const int chunk = std::min(256, std::max(8, ncell / (4 * 8 * 148)));
+  lists_sort_kernel<T><<<unsigned((ncell + chunk - 1ll) / chunk), 256, 0, st>>>(start, count, ncell, chunk, list);
   int rc = check_launch("lists_sort_kernel");
   if (rc) return rc;
   size_t bytes = 0;
@@ -273,8 +297,9 @@ int sort_lists(const int* start, const int* count, int ncell, int S, T* list, cu
   if (cudaFuncSetAttribute(long_lists_sort_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            kBitmapKeys / 8) != cudaSuccess)
     return check_launch("long_lists_sort_kernel attribute");
-  const int ctas = (ncell + 255) / 256 < 148 * 4 ? (ncell + 255) / 256 : 148 * 4;
-  long_lists_sort_kernel<T><<<unsigned(ctas), 256, bytes, st>>>(start, count, ncell, S, list);
+  const int most = 148 * 4, per = std::min(256, (ncell - 1) / most + 1);
+  const int ctas = std::min(most, (ncell - 1) / per + 1);
+  long_lists_sort_kernel<T><<<unsigned(ctas), 256, bytes, st>>>(start, count, ncell, per, S, list);
   return check_launch("long_lists_sort_kernel");
 }
 

@@ -4,9 +4,11 @@ import subprocess
 import sys
 from pathlib import Path
 
+import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
 
 ROOT = Path(__file__).resolve().parents[1]
 
@@ -38,3 +40,29 @@ print("built")
 def test_lists_of_a_fresh_process():
     r = subprocess.run([sys.executable, "-c", FRESH], cwd=ROOT, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and "built" in r.stdout, r.stderr[-800:]
+
+
+# both sides of the bitmap's number of keys; lists of more than 128 entries in
+# every cell, and in one cell of many empty ones; a grid of empty cells
+@pytest.mark.parametrize("S,nseg,spread", [(1 << 20, 12, 20.0), ((1 << 20) + 1, 12, 20.0), ((1 << 20) + 1, 90, 20.0),
+                                           (5000, 130, 0.5), (3, 130, 20.0)])
+def test_sorted_lists(S, nseg, spread):
+    from nozomi_b200 import engine
+    rng = np.random.default_rng(S)
+    sph = np.zeros((5, S))
+    sph[:3] = rng.uniform(-spread, spread, (3, S))
+    sph[3] = 0.1
+    sph[4] = rng.integers(0, 3, S)
+    sub = engine.DeviceSubstrate(sph, 3, (40.0,) * 3, (nseg,) * 3, np.full(4, 2.0), np.full(4, 80.0), jump_tol=0.2)
+    n = sub.n_items
+    start, count, items, idx = (t.cpu().numpy() for t in (sub.cell_start, sub.cell_count, sub.cell_items[:n],
+                                                          sub.cell_idx[:n]))
+    assert np.array_equal(start, np.cumsum(count) - count) and count.sum() == n
+    inner = np.ones(n, bool)  # entries that follow one of the same cell
+    inner[start[count > 0]] = False
+    assert (np.diff(items)[inner[1:]] > 0).all()
+    idx = idx.astype(np.int64) & (0xFFFF if sub.idx_bytes == 2 else 0xFFFFFFFF)
+    assert (np.diff(idx)[inner[1:]] > 0).all()
+    cell = np.repeat(np.arange(count.size, dtype=np.int64), count)
+    want = cell * S + sub.perm.cpu().numpy()[items]
+    assert np.array_equal(np.sort(want), cell * S + idx)
