@@ -30,19 +30,22 @@ struct CellGeom {
   double tol;
 };
 
-// Valid cell range [lo, hi] on one axis (empty when lo > hi), by the lanes of
-// a warp, a candidate cell each.
-__device__ __forceinline__ void axis_range_warp(double x, double r, double L, int nseg, double tol, int lane, int& lo,
-                                                int& hi) {
+// Valid cell range [lo, hi] on one axis (empty when lo > hi, and for a lane
+// that is not live), by each G lanes of a warp, a candidate cell a lane.
+template <int G>
+__device__ __forceinline__ void axis_range(bool live, double x, double r, double L, int nseg, double tol, int lane,
+                                           int& lo, int& hi) {
   const double dL = L / nseg;
   const int a = max(int(floor((x - r + L / 2 - tol) / dL)) - 2, 0);
-  const int b = min(int(ceil((tol + r + x + L / 2) / dL)) + 2, nseg - 1);
+  const int b = live ? min(int(ceil((tol + r + x + L / 2) / dL)) + 2, nseg - 1) : -1;
   lo = 1;
   hi = 0;
-  for (int base = a; base <= b; base += 32) {
-    const int n = base + lane;
-    const unsigned ok = __ballot_sync(
-        0xffffffffu, n <= b && seg_lo(double(n), dL, r, x, L) < tol && seg_hi(double(n), dL, r, x, L) < tol);
+  for (int base = a; __any_sync(0xffffffffu, base <= b); base += G) {
+    const int n = base + lane % G;
+    const unsigned ok = __ballot_sync(0xffffffffu, n <= b && seg_lo(double(n), dL, r, x, L) < tol &&
+                                                       seg_hi(double(n), dL, r, x, L) < tol) >>
+                            (lane & ~(G - 1)) &
+                        (0xffffffffu >> (32 - G));
     if (ok) {
       if (lo > hi) lo = base + __ffs(ok) - 1;
       hi = base + 31 - __clz(ok);
@@ -70,42 +73,79 @@ __device__ __forceinline__ bool within_round(double x, double y, double z, doubl
   return ex * ex + ey * ey + ez * ez <= R * R;
 }
 
-// The cells of every sphere, counted (items null) or filled in: a warp per
-// sphere, its lanes over the cells of the sphere's box (hundreds for small
-// cells), so that the lanes' atomics fall on neighbouring counters.  Bound by
-// the atomics: 80,000 spheres in 420,000 cells (24 M members) are counted and
-// filled in in 0.30 ms, 0.53 ms by one thread a sphere.
-template <bool ROUND>
+// The cells of every sphere, counted (items null) or filled in: G lanes a
+// sphere, over the cells of its box, so that their atomics fall on
+// neighbouring counters.  Bound by the atomics, and for many spheres in few
+// cells each by the double-precision ranges, which every lane of a sphere
+// forms (a warp a sphere took 0.60 ms to count 1.1e6 spheres of 23 cells, two
+// lanes 0.11).
+template <bool ROUND, int G>
 __global__ void __launch_bounds__(256) cells_members_kernel(const double* __restrict__ sph, int S, CellGeom g,
                                                             const int* __restrict__ offsets, int* __restrict__ cursor,
                                                             int* __restrict__ items) {
-  const int s = int((blockIdx.x * size_t(blockDim.x) + threadIdx.x) >> 5), lane = threadIdx.x & 31;
-  if (s >= S) return;
+  const size_t at = (blockIdx.x * size_t(blockDim.x) + threadIdx.x) / G;
+  const bool live = at < size_t(S);
+  const int s = live ? int(at) : 0, lane = threadIdx.x & 31;
   const double x = sph[s], y = sph[size_t(S) + s], z = sph[2 * size_t(S) + s], r = sph[3 * size_t(S) + s];
   int x0, x1, y0, y1, z0, z1;
-  axis_range_warp(x, r, g.Lx, g.nx, g.tol, lane, x0, x1);
-  axis_range_warp(y, r, g.Ly, g.ny, g.tol, lane, y0, y1);
-  axis_range_warp(z, r, g.Lz, g.nz, g.tol, lane, z0, z1);
+  axis_range<G>(live, x, r, g.Lx, g.nx, g.tol, lane, x0, x1);
+  axis_range<G>(live, y, r, g.Ly, g.ny, g.tol, lane, y0, y1);
+  axis_range<G>(live, z, r, g.Lz, g.nz, g.tol, lane, z0, z1);
   if (x0 > x1 || y0 > y1 || z0 > z1) return;
-  const unsigned X = unsigned(x1 - x0 + 1), Y = unsigned(y1 - y0 + 1);
-  const unsigned long long total = 1ull * X * Y * unsigned(z1 - z0 + 1);
-  for (unsigned long long t = lane; t < total; t += 32) {
-    unsigned row, n, p, m;
-    if (total <= 0xffffffffull) {
-      row = unsigned(t) / X;
-      n = unsigned(t) - row * X;
-    } else {
-      row = unsigned(t / X);
-      n = unsigned(t - 1ull * row * X);
-    }
-    p = row / Y;
-    m = row - p * Y;
-    const int cn = x0 + int(n), cm = y0 + int(m), cp = z0 + int(p);
-    if (ROUND && !within_round(x, y, z, r, g, cn, cm, cp)) continue;
-    const size_t c = (size_t(cp) * g.ny + cm) * g.nx + cn;
+  auto add = [&](int n, int m, int p) {
+    if (ROUND && !within_round(x, y, z, r, g, n, m, p)) return;
+    const size_t c = (size_t(p) * g.ny + m) * g.nx + n;
     const int slot = atomicAdd(cursor + c, 1);
     if (items) items[offsets[c] + slot] = s;
+  };
+  const unsigned Y = unsigned(y1 - y0 + 1), Z = unsigned(z1 - z0 + 1);
+  const unsigned first = lane % G;
+  if (ROUND && G <= 2) {  // a lane takes every G-th row: the distances in y and z are formed once a row
+    unsigned m = first % Y, p = first / Y;
+    while (p < Z) {
+      for (int n = x0; n <= x1; ++n) add(n, y0 + int(m), z0 + int(p));
+      m += G;
+      while (m >= Y) {
+        m -= Y;
+        ++p;
+      }
+    }
+    return;
   }
+  // every G-th cell of the box: the lane's first, and the step of G, as digits
+  const unsigned X = unsigned(x1 - x0 + 1);
+  unsigned n = first % X, m = first / X % Y, p = first / X / Y;
+  const unsigned dn = G % X, dm = G / X % Y, dp = G / X / Y;
+  while (p < Z) {
+    add(x0 + int(n), y0 + int(m), z0 + int(p));
+    n += dn;
+    m += dm;
+    p += dp;
+    if (n >= X) {
+      n -= X;
+      ++m;
+    }
+    if (m >= Y) {
+      m -= Y;
+      ++p;
+    }
+  }
+}
+
+template <bool ROUND>
+int cells_members(const double* sph, int S, const CellGeom& g, const int* offsets, int* cursor, int* items,
+                  cudaStream_t st) {
+  auto launch = [&](auto kernel, int lanes) {
+    kernel<<<unsigned((size_t(S) * lanes + 255) / 256), 256, 0, st>>>(sph, S, g, offsets, cursor, items);
+  };
+  // lanes a sphere: many while spheres alone do not fill the GPU.  Counted, one
+  // thread a sphere / 2 / 8 / 32 lanes: 6,000 spheres of 450 cells 0.091 /
+  // 0.040 / 0.021 / 0.019 ms, 80,000 of 247 0.159 / 0.103 / 0.056 / 0.079,
+  // 3e5 of 8 0.076 / 0.050 / 0.058 / 0.177, 1e6 of 4 0.110 / 0.080 / 0.152 / 0.542.
+  if (S <= 16384) launch(cells_members_kernel<ROUND, 32>, 32);
+  else if (S <= 524288) launch(cells_members_kernel<ROUND, 8>, 8);
+  else launch(cells_members_kernel<ROUND, 2>, 2);
+  return check_launch("cells_members_kernel");
 }
 
 // Ascending order within each cell's list, keys in [0, S).  A warp per list of
@@ -992,9 +1032,7 @@ extern "C" int nz_cells_count(const double* spheres64, int S, double Lx, double 
   if (cudaMemsetAsync(counts, 0, ncell * sizeof(int), st) != cudaSuccess) return check_launch("nz_cells_count memset");
   if (S == 0) return NZ_OK;
   CellGeom g{Lx, Ly, Lz, nx, ny, nz_, jump_tol};
-  cells_members_kernel<false><<<unsigned((size_t(S) * 32 + 255) / 256), 256, 0, st>>>(spheres64, S, g, nullptr, counts,
-                                                                                   nullptr);
-  return check_launch("cells_members_kernel");
+  return cells_members<false>(spheres64, S, g, nullptr, counts, nullptr, st);
 }
 
 extern "C" int nz_cells_count_round(const double* spheres64, int S, double Lx, double Ly, double Lz, int nx, int ny,
@@ -1007,9 +1045,7 @@ extern "C" int nz_cells_count_round(const double* spheres64, int S, double Lx, d
     return check_launch("nz_cells_count_round memset");
   if (S == 0) return NZ_OK;
   CellGeom g{Lx, Ly, Lz, nx, ny, nz_, margin};
-  cells_members_kernel<true><<<unsigned((size_t(S) * 32 + 255) / 256), 256, 0, st>>>(spheres64, S, g, nullptr, counts,
-                                                                                  nullptr);
-  return check_launch("cells_members_kernel");
+  return cells_members<true>(spheres64, S, g, nullptr, counts, nullptr, st);
 }
 
 extern "C" int nz_cells_fill_round(const double* spheres64, int S, double Lx, double Ly, double Lz, int nx, int ny,
@@ -1024,9 +1060,7 @@ extern "C" int nz_cells_fill_round(const double* spheres64, int S, double Lx, do
     return check_launch("nz_cells_fill_round memset");
   if (S == 0) return NZ_OK;
   CellGeom g{Lx, Ly, Lz, nx, ny, nz_, margin};
-  cells_members_kernel<true><<<unsigned((size_t(S) * 32 + 255) / 256), 256, 0, st>>>(spheres64, S, g, offsets, cursor,
-                                                                                    items);
-  int rc = check_launch("cells_members_kernel");
+  int rc = cells_members<true>(spheres64, S, g, offsets, cursor, items, st);
   if (rc != NZ_OK) return rc;
   return sort_lists(offsets, counts, int(ncell), S, items, st);
 }
@@ -1065,9 +1099,7 @@ extern "C" int nz_cells_fill(const double* spheres64, int S, double Lx, double L
   if (cudaMemsetAsync(cursor, 0, ncell * sizeof(int), st) != cudaSuccess) return check_launch("nz_cells_fill memset");
   if (S == 0) return NZ_OK;
   CellGeom g{Lx, Ly, Lz, nx, ny, nz_, jump_tol};
-  cells_members_kernel<false><<<unsigned((size_t(S) * 32 + 255) / 256), 256, 0, st>>>(spheres64, S, g, offsets, cursor,
-                                                                                    items);
-  int rc = check_launch("cells_members_kernel");
+  int rc = cells_members<false>(spheres64, S, g, offsets, cursor, items, st);
   if (rc != NZ_OK) return rc;
   return sort_lists(offsets, counts, int(ncell), S, items, st);
 }

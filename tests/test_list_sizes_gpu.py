@@ -66,3 +66,30 @@ def test_sorted_lists(S, nseg, spread):
     cell = np.repeat(np.arange(count.size, dtype=np.int64), count)
     want = cell * S + sub.perm.cpu().numpy()[items]
     assert np.array_equal(np.sort(want), cell * S + idx)
+
+
+# both sides of each number of lanes a sphere: the counts of all spheres are
+# the sums of the counts of short runs of them (pinned to the oracle in
+# test_lists_gpu.py), for boxes of one cell to hundreds
+@pytest.mark.parametrize("S", [16384, 16385, 524288, 524289])
+@pytest.mark.parametrize("nseg", [(1, 1, 1), (5, 3, 40), (61, 60, 59)])
+def test_members_by_lanes(S, nseg):
+    import ctypes
+    from nozomi_b200 import _lib as L
+    lib = L.load()
+    rng = np.random.default_rng(S)
+    box, ncell = (24.0, 25.0, 26.0), nseg[0] * nseg[1] * nseg[2]
+    sph = np.zeros((5, S))
+    sph[:3] = rng.uniform(-0.6, 0.6, (3, S)) * np.asarray(box)[:, None]
+    sph[3] = rng.uniform(0.0, 0.9, S)
+    p = lambda t: ctypes.c_void_p(t.data_ptr())  # noqa: E731
+
+    def counts(fn, part):
+        d = torch.from_numpy(np.ascontiguousarray(part)).cuda()
+        c = torch.empty(ncell, dtype=torch.int32, device="cuda")
+        L.check(fn(p(d), part.shape[1], *box, *nseg, 0.3, p(c), None), "count")
+        return c.cpu().numpy()
+
+    for fn in (lib.nz_cells_count, lib.nz_cells_count_round):
+        want = sum(counts(fn, sph[:, i:i + 16000]) for i in range(0, S, 16000))
+        np.testing.assert_array_equal(counts(fn, sph), want)
