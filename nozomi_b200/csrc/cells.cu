@@ -231,8 +231,11 @@ __global__ void __launch_bounds__(256) lists_sort_kernel(const int* __restrict__
 // of the S keys in shared memory and reads them back in order, unless they
 // ascend already.  CTAs look over `chunk` cells at a time, few enough that a
 // coarse grid's lists reach every SM.  Lists with repeats are heapsorted by
-// one thread; with more keys than the bitmap holds every thread heapsorts a
-// list.
+// one thread.  With more keys than the bitmap holds, a CTA sorts a list of up
+// to kSharedSort entries in shared memory by a bitonic network, and beyond
+// that each thread heapsorts a list.  1.1e6 spheres with lists of 564: the
+// heapsorts, a thread each, took 2.9 ms from entries almost in order and 4.2
+// from the order that cells_members_kernel leaves; the network 0.38 ms.
 template <typename T>
 __device__ void heapsort(T* a, int n) {
   auto sift = [&](int root, int end) {
@@ -256,27 +259,19 @@ __device__ void heapsort(T* a, int n) {
 }
 
 constexpr int kBitmapKeys = 1 << 20;  // 128 KiB of shared memory
+constexpr int kSharedSort = 1 << 13;  // 32 KiB: seven CTAs an SM
 
 template <typename T>
 __global__ void __launch_bounds__(256) long_lists_sort_kernel(const int* __restrict__ start,
                                                               const int* __restrict__ count, int ncell, int chunk,
                                                               int S, T* __restrict__ list) {
-  extern __shared__ unsigned s_bits[];  // (S + 31) / 32 words, or none beyond kBitmapKeys keys
+  extern __shared__ unsigned s_bits[];  // (S + 31) / 32 words, or kSharedSort keys
   __shared__ int s_cells[256];
   __shared__ int s_n, s_repeats, s_before[8];
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const int words = (S + 31) / 32;
   for (long long base = 1ll * blockIdx.x * chunk; base < ncell; base += 1ll * gridDim.x * chunk) {
     const bool is_long = t < chunk && base + t < ncell && count[base + t] > kWarpSort;
-    if (S > kBitmapKeys) {
-      if (!is_long) continue;
-      T* a = list + start[base + t];
-      const int n = count[base + t];
-      int i = 1;
-      while (i < n && a[i - 1] <= a[i]) ++i;
-      if (i < n) heapsort(a, n);
-      continue;
-    }
     __syncthreads();
     if (t == 0) s_n = 0;
     __syncthreads();
@@ -289,6 +284,29 @@ __global__ void __launch_bounds__(256) long_lists_sort_kernel(const int* __restr
       bool sorted = true;
       for (int i = t + 1; i < n; i += 256) sorted &= a[i - 1] <= a[i];
       if (__syncthreads_and(sorted)) continue;
+      if (S > kBitmapKeys) {
+        if (n > kSharedSort) continue;
+        int* const v = reinterpret_cast<int*>(s_bits);
+        int size2 = 2 * kWarpSort;
+        while (size2 < n) size2 *= 2;
+        for (int i = t; i < size2; i += 256) v[i] = i < n ? int(a[i]) : 0x7fffffff;
+        for (int size = 2; size <= size2; size *= 2)
+          for (int stride = size / 2; stride > 0; stride /= 2) {
+            __syncthreads();
+            for (int i = t; i < size2 / 2; i += 256) {
+              const int k = 2 * i - (i & (stride - 1)), o = k + stride;
+              const int x = v[k], y = v[o];
+              if ((x > y) == ((k & size) == 0)) {
+                v[k] = y;
+                v[o] = x;
+              }
+            }
+          }
+        __syncthreads();
+        for (int i = t; i < n; i += 256) a[i] = T(v[i]);
+        __syncthreads();
+        continue;
+      }
       for (int w = t; w < words; w += 256) s_bits[w] = 0u;
       if (t == 0) s_repeats = 0;
       __syncthreads();
@@ -320,6 +338,13 @@ __global__ void __launch_bounds__(256) long_lists_sort_kernel(const int* __restr
         for (unsigned b = s_bits[w]; b; b &= b - 1) a[at++] = T(32 * w + __ffs(b) - 1);
       __syncthreads();
     }
+    if (S > kBitmapKeys && is_long && count[base + t] > kSharedSort) {
+      T* a = list + start[base + t];
+      const int n = count[base + t];
+      int i = 1;
+      while (i < n && a[i - 1] <= a[i]) ++i;
+      if (i < n) heapsort(a, n);
+    }
   }
 }
 
@@ -331,8 +356,7 @@ int sort_lists(const int* start, const int* count, int ncell, int S, T* list, cu
   lists_sort_kernel<T><<<unsigned((ncell + chunk - 1ll) / chunk), 256, 0, st>>>(start, count, ncell, chunk, list);
   int rc = check_launch("lists_sort_kernel");
   if (rc) return rc;
-  size_t bytes = 0;
-  if (S <= kBitmapKeys) bytes = size_t((S + 31) / 32) * sizeof(unsigned);
+  const size_t bytes = S <= kBitmapKeys ? size_t((S + 31) / 32) * sizeof(unsigned) : kSharedSort * sizeof(int);
   // at every size: the 48 KiB allowed without it are for static and dynamic bytes together
   if (cudaFuncSetAttribute(long_lists_sort_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            kBitmapKeys / 8) != cudaSuccess)

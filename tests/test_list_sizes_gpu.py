@@ -45,6 +45,7 @@ def test_lists_of_a_fresh_process():
 # both sides of the bitmap's number of keys; lists of more than 128 entries in
 # every cell, and in one cell of many empty ones; a grid of empty cells
 @pytest.mark.parametrize("S,nseg,spread", [(1 << 20, 12, 20.0), ((1 << 20) + 1, 12, 20.0), ((1 << 20) + 1, 90, 20.0),
+                                           ((1 << 20) + 1, 5, 20.0), ((1 << 20) + 1, 6, 20.0),
                                            (5000, 130, 0.5), (3, 130, 20.0)])
 def test_sorted_lists(S, nseg, spread):
     from nozomi_b200 import engine
