@@ -377,11 +377,13 @@ __device__ __forceinline__ unsigned long long okey(double v) {
 // distances, two per axis; a CTA takes up to kSegCells cells of one row
 // (same m, p), so the y and z distances of a sphere are formed once for all
 // of them.  The K spheres of least (in_segment, index) of each cell:
-//   1. a histogram of the distances, in single precision, over kSegBuckets
-//      equal steps finds the step of the K-th.  The K-th smallest of the true
-//      distances differs from the K-th smallest of these by no more than
-//      their rounding, and a step (1.5e-3 of the box) is thousands of
-//      roundings wide: spheres two steps below are in, two steps above out;
+//   1. a histogram of the distances over kSegBuckets equal steps finds the
+//      step of the K-th.  A sphere's distances from the row and from the
+//      row's first cell are formed in double precision (a sphere far larger
+//      than the box, a flat wall, is the difference of two large numbers),
+//      rounded, and moved from cell to cell in single precision: within the
+//      steps the roundings are a thousandth of one (1.5e-3 of the box), so
+//      spheres two steps below the K-th are in, two steps above out;
 //   2. the spheres of the three steps between, a few tens, are collected and
 //      ranked by their exact double-precision keys (a radix select over them
 //      when there are more than kSegCandidates: many equal distances);
@@ -433,22 +435,27 @@ __global__ void __launch_bounds__(256, 3) segments_fill_kernel(const double* __r
     return;
   }
   const double dLx = g.Lx / g.nx, dLy = g.Ly / g.ny, dLz = g.Lz / g.nz;
-  // single precision, for the steps: half a cell and the cell's centre
-  const float hx = float(0.5 * dLx), hy = float(0.5 * dLy), hz = float(0.5 * dLz);
-  const float oy = float((m + 0.5) * dLy - g.Ly / 2), oz = float((p + 0.5) * dLz - g.Lz / 2);
+  // for the steps: half a cell, the centres of the row and of its first cell
+  const float hx = float(0.5 * dLx), hy = float(0.5 * dLy), hz = float(0.5 * dLz), fx = float(dLx);
+  const double oy = (m + 0.5) * dLy - g.Ly / 2, oz = (p + 0.5) * dLz - g.Lz / 2, ox = (n0 + 0.5) * dLx - g.Lx / 2;
   const float span = float(fmax(g.Lx, fmax(g.Ly, g.Lz)));
   const float scale = float(kSegBuckets) / (1.5f * span);
-  auto step_of = [&](float v) {  // (v + span / 2) * scale; ascending in v
-    return __float2int_rd(fminf(float(kSegBuckets - 1), fmaxf(0.0f, __fmaf_rn(v, scale, kSegBuckets / 3.0f))));
+  auto step_of = [&](float v) {  // (v + span / 2) * scale; ascending in v, NaN last as its key
+    return __float2int_rd(fmaxf(0.0f, fminf(float(kSegBuckets - 1), __fmaf_rn(v, scale, kSegBuckets / 3.0f))));
   };
-  auto yz_step = [&](int i, float& yz, float& r) {
-    r = float(sph[3 * size_t(S) + i]);
-    yz = fmaxf(fabsf(float(sph[size_t(S) + i]) - oy) - hy, fabsf(float(sph[2 * size_t(S) + i]) - oz) - hz) - r;
+  auto yz_step = [&](int i, float& yz) {
+    const double r = sph[3 * size_t(S) + i];
+    yz = fmaxf(float(fabs(sph[size_t(S) + i] - oy) - r) - hy, float(fabs(sph[2 * size_t(S) + i] - oz) - r) - hz);
     return step_of(yz);
   };
-  auto step_in = [&](int i, int c, float yz, float r) {
-    const float ox = float((n0 + c + 0.5) * dLx - g.Lx / 2);
-    return step_of(fmaxf(yz, fabsf(float(sph[i]) - ox) - hx - r));
+  auto x_ends = [&](int i, float& xl, float& xh) {  // both sides' distances from the first cell's centre
+    const double x = sph[i] - ox, r = sph[3 * size_t(S) + i];
+    xl = float(x - r);
+    xh = float(-x - r);
+  };
+  auto step_in = [&](int c, float yz, float xl, float xh) {
+    const float at = c * fx;
+    return step_of(fmaxf(yz, fmaxf(xl - at, xh + at) - hx));
   };
   auto key_of = [&](int i, int c) {  // exact: the reference's in_segment, operation by operation
     const double r = sph[3 * size_t(S) + i];
@@ -487,10 +494,11 @@ __global__ void __launch_bounds__(256, 3) segments_fill_kernel(const double* __r
     __syncthreads();
     for (int k = t * stride; k < len; k += blockDim.x * stride) {
       const int i = sphere(k);
-      float yz, r;
-      if (yz_step(i, yz, r) > limit) continue;
+      float yz, xl, xh;
+      if (yz_step(i, yz) > limit) continue;
+      x_ends(i, xl, xh);
       for (int c = 0; c < nc; ++c) {
-        const int b = step_in(i, c, yz, r);
+        const int b = step_in(c, yz, xl, xh);
         if (b <= limit) atomicAdd(&sm.hist[c][b], 1);
       }
     }
@@ -503,8 +511,8 @@ __global__ void __launch_bounds__(256, 3) segments_fill_kernel(const double* __r
 #pragma unroll 4
     for (int w = warp; w < words; w += 8) {
       const int i = 32 * w + lane;
-      float yz, r;
-      const unsigned mask = __ballot_sync(0xffffffffu, i < S && yz_step(min(i, S - 1), yz, r) <= limit);
+      float yz;
+      const unsigned mask = __ballot_sync(0xffffffffu, i < S && yz_step(min(i, S - 1), yz) <= limit);
       if (lane == 0) bits[w] = mask;
     }
     __syncthreads();
@@ -577,11 +585,12 @@ __global__ void __launch_bounds__(256, 3) segments_fill_kernel(const double* __r
   // 2. the exact key of the K-th
   for (int k = t; k < len; k += blockDim.x) {
     const int i = sphere(k);
-    float yz, r;
-    if (yz_step(i, yz, r) > limit) continue;
+    float yz, xl, xh;
+    if (yz_step(i, yz) > limit) continue;
+    x_ends(i, xl, xh);
     for (int c = 0; c < nc; ++c) {
       const int step = s_cell[c].step;
-      if (s_cell[c].count > kSegCandidates || abs(step_in(i, c, yz, r) - step) > 1) continue;
+      if (s_cell[c].count > kSegCandidates || abs(step_in(c, yz, xl, xh) - step) > 1) continue;
       sm.keys[c][atomicAdd(&s_n[c], 1)] = key_of(i, c);
     }
   }
@@ -617,8 +626,10 @@ __global__ void __launch_bounds__(256, 3) segments_fill_kernel(const double* __r
       __syncthreads();
       for (int j = t; j < len; j += blockDim.x) {
         const int i = sphere(j);
-        float yz, r;
-        if (yz_step(i, yz, r) > limit || abs(step_in(i, c, yz, r) - q.step) > 1) continue;
+        float yz, xl, xh;
+        if (yz_step(i, yz) > limit) continue;
+        x_ends(i, xl, xh);
+        if (abs(step_in(c, yz, xl, xh) - q.step) > 1) continue;
         const unsigned long long k = key_of(i, c);
         if ((k & mask) == prefix) atomicAdd(&hist[(k >> (8 * digit)) & 255ull], 1);
       }
@@ -639,8 +650,8 @@ __global__ void __launch_bounds__(256, 3) segments_fill_kernel(const double* __r
   // 3. a run of the passes' spheres per warp: count, then write in order
   const int run = (len + 255) / 256 * 32;
   const int k0 = min(len, warp * run), k1 = min(len, k0 + run);
-  auto classify = [&](int i, int c, float yz, float r, bool& less, bool& tie) {
-    const int d = step_in(i, c, yz, r) - s_cell[c].step;
+  auto classify = [&](int i, int c, float yz, float xl, float xh, bool& less, bool& tie) {
+    const int d = step_in(c, yz, xl, xh) - s_cell[c].step;
     less = d < -1;
     tie = false;
     if (d >= -1 && d <= 1) {
@@ -654,14 +665,15 @@ __global__ void __launch_bounds__(256, 3) segments_fill_kernel(const double* __r
   for (int c = 0; c < kSegCells; ++c) less_n[c] = tie_n[c] = 0;
   for (int base = k0; base < k1; base += 32) {
     const int i = base + lane < k1 ? sphere(base + lane) : -1;
-    float yz, r;
-    const bool live = i >= 0 && yz_step(i, yz, r) <= limit;
+    float yz, xl, xh;
+    const bool live = i >= 0 && yz_step(i, yz) <= limit;
     if (!__any_sync(0xffffffffu, live)) continue;
+    if (live) x_ends(i, xl, xh);
 #pragma unroll
     for (int c = 0; c < kSegCells; ++c) {
       if (c >= nc) break;
       bool less = false, tie = false;
-      if (live) classify(i, c, yz, r, less, tie);
+      if (live) classify(i, c, yz, xl, xh, less, tie);
       less_n[c] += __popc(__ballot_sync(0xffffffffu, less));
       tie_n[c] += __popc(__ballot_sync(0xffffffffu, tie));
     }
@@ -687,14 +699,15 @@ __global__ void __launch_bounds__(256, 3) segments_fill_kernel(const double* __r
   }
   for (int base = k0; base < k1; base += 32) {
     const int i = base + lane < k1 ? sphere(base + lane) : -1;
-    float yz, r;
-    const bool live = i >= 0 && yz_step(i, yz, r) <= limit;
+    float yz, xl, xh;
+    const bool live = i >= 0 && yz_step(i, yz) <= limit;
     if (!__any_sync(0xffffffffu, live)) continue;
+    if (live) x_ends(i, xl, xh);
 #pragma unroll
     for (int c = 0; c < kSegCells; ++c) {
       if (c >= nc) break;
       bool less = false, tie = false;
-      if (live) classify(i, c, yz, r, less, tie);
+      if (live) classify(i, c, yz, xl, xh, less, tie);
       const unsigned tb = __ballot_sync(0xffffffffu, tie);
       const bool take = less || (tie && ties[c] + __popc(tb & lower) < s_cell[c].rank);
       ties[c] += __popc(tb);
