@@ -385,8 +385,11 @@ __device__ __forceinline__ unsigned long long okey(double v) {
 //      steps the roundings are a thousandth of one (1.5e-3 of the box), so
 //      spheres two steps below the K-th are in, two steps above out;
 //   2. the spheres of the three steps between, a few tens, are collected and
-//      ranked by their exact double-precision keys (a radix select over them
-//      when there are more than kSegCandidates: many equal distances);
+//      ranked by their exact double-precision keys.  Beyond kSegCandidates
+//      (cells of hundreds of spheres, equal distances) a radix select over
+//      the collected keys takes over, or over the passes' spheres when shared
+//      memory does not hold the keys: 1e5 spheres in 3^3 cells, 8,412 a cell,
+//      take 1.21 ms, 2.86 with the keys formed anew for each digit;
 //   3. two passes in index order count and write the chosen ones, a run of
 //      spheres per warp, ties to the lower index.
 // A sixteenth of the spheres, looked at first, gives a step that almost
@@ -398,6 +401,7 @@ __device__ __forceinline__ unsigned long long okey(double v) {
 // ten double-precision passes over all spheres (8-bit radix select, then the
 // output), 0.37 ms so.
 constexpr int kSegCells = 8, kSegBuckets = 1024, kSegCandidates = 256, kSegSample = 16;
+constexpr int kSegKeys = kSegCells * kSegBuckets / 2;  // keys that fit where the histograms were
 constexpr int kSegKept = 4096;          // spheres noted for the later passes
 constexpr int kSegBitmap = 262144;      // spheres up to which they are noted
 
@@ -416,8 +420,9 @@ __global__ void __launch_bounds__(256, 3) segments_fill_kernel(const double* __r
                                                             int per, int* __restrict__ segments) {
   __shared__ union {
     int hist[kSegCells][kSegBuckets];
-    unsigned long long keys[kSegCells][kSegCandidates];
+    unsigned long long keys[kSegKeys];
   } sm;
+  __shared__ int s_digit[256];
   __shared__ SegCell s_cell[kSegCells];
   __shared__ int s_n[kSegCells];
   __shared__ int s_less[8][kSegCells], s_tie[8][kSegCells];
@@ -466,11 +471,11 @@ __global__ void __launch_bounds__(256, 3) segments_fill_kernel(const double* __r
                               g.Lz / 2));
     return okey(v);
   };
-  // the step at which a histogram's running count reaches `target` (warp c
-  // for cell c), or kSegBuckets; `before`: the count up to two steps below it
-  auto reach = [&](const int* hist, int target) {
-    int run = 0;
-    for (int base = 0; base < kSegBuckets; base += 32) {
+  // the step at which a histogram's running count reaches `target`, or
+  // `steps`, by a warp; `run`: the count before it
+  auto reach = [&](const int* hist, int steps, int target, int& run) {
+    run = 0;
+    for (int base = 0; base < steps; base += 32) {
       int incl = hist[base + lane];
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
@@ -478,10 +483,14 @@ __global__ void __launch_bounds__(256, 3) segments_fill_kernel(const double* __r
         if (lane >= o) incl += v;
       }
       const unsigned reached = __ballot_sync(0xffffffffu, run + incl >= target);
-      if (reached) return base + __ffs(reached) - 1;
+      if (reached) {
+        const int b = __ffs(reached) - 1;
+        run += __shfl_sync(0xffffffffu, incl - hist[base + lane], b);
+        return base + b;
+      }
       run += __shfl_sync(0xffffffffu, incl, 31);
     }
-    return kSegBuckets;
+    return steps;
   };
   const unsigned lower = (1u << lane) - 1u;
   int len = S;  // the passes' spheres: all, or the first len entries of s_kept
@@ -547,7 +556,8 @@ __global__ void __launch_bounds__(256, 3) segments_fill_kernel(const double* __r
     if (t == 0) s_limit = 0;
     __syncthreads();
     if (warp < nc) {
-      const int b = reach(sm.hist[warp], 2 * (K / kSegSample) + 8);
+      int before;
+      const int b = reach(sm.hist[warp], kSegBuckets, 2 * (K / kSegSample) + 8, before);
       if (lane == 0) atomicMax(&s_limit, b);
     }
     __syncthreads();
@@ -559,11 +569,9 @@ __global__ void __launch_bounds__(256, 3) segments_fill_kernel(const double* __r
     if (t == 0) s_limit = 0;
     __syncthreads();
     if (warp < nc) {
-      const int b = reach(sm.hist[warp], K);
-      int below = 0;
-      for (int k = lane; k < b - 1; k += 32) below += sm.hist[warp][k];
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) below += __shfl_xor_sync(0xffffffffu, below, o);
+      int below;
+      const int b = reach(sm.hist[warp], kSegBuckets, K, below);
+      if (b > 0) below -= sm.hist[warp][b - 1];  // up to two steps below the K-th's
       if (lane == 0) {
         SegCell& q = s_cell[warp];
         q.step = b;
@@ -583,6 +591,7 @@ __global__ void __launch_bounds__(256, 3) segments_fill_kernel(const double* __r
   limit = min(limit, s_limit);
 
   // 2. the exact key of the K-th
+  const int room = kSegKeys / per;  // keys of a cell
   for (int k = t; k < len; k += blockDim.x) {
     const int i = sphere(k);
     float yz, xl, xh;
@@ -590,20 +599,21 @@ __global__ void __launch_bounds__(256, 3) segments_fill_kernel(const double* __r
     x_ends(i, xl, xh);
     for (int c = 0; c < nc; ++c) {
       const int step = s_cell[c].step;
-      if (s_cell[c].count > kSegCandidates || abs(step_in(c, yz, xl, xh) - step) > 1) continue;
-      sm.keys[c][atomicAdd(&s_n[c], 1)] = key_of(i, c);
+      if (s_cell[c].count > room || abs(step_in(c, yz, xl, xh) - step) > 1) continue;
+      sm.keys[c * room + atomicAdd(&s_n[c], 1)] = key_of(i, c);
     }
   }
   __syncthreads();
-  if (warp < nc) {  // each candidate: how many are less, how many equal
+  if (warp < nc && s_n[warp] <= kSegCandidates) {  // each candidate: how many are less, how many equal
     const int n = s_n[warp], rank = s_cell[warp].rank;
+    const unsigned long long* const keys = sm.keys + warp * room;
     __syncwarp();
     for (int i = lane; i < n; i += 32) {
-      const unsigned long long k = sm.keys[warp][i];
+      const unsigned long long k = keys[i];
       int less = 0, same = 0;
       for (int j = 0; j < n; ++j) {
-        less += sm.keys[warp][j] < k;
-        same += sm.keys[warp][j] == k;
+        less += keys[j] < k;
+        same += keys[j] == k;
       }
       if (less < rank && rank <= less + same) {  // every candidate equal to the K-th writes the same
         s_cell[warp].key = k;
@@ -617,25 +627,29 @@ __global__ void __launch_bounds__(256, 3) segments_fill_kernel(const double* __r
   for (int c = 0; c < nc; ++c) {  // many spheres around the K-th: radix select by 8 bits over them
     const SegCell q = s_cell[c];
     if (q.count <= kSegCandidates) continue;
+    const bool held = q.count <= room;  // their keys were collected
     unsigned long long prefix = 0ull, mask = 0ull;
     int rank = q.rank;
-    int* const hist = sm.hist[0];
     for (int digit = 7; digit >= 0; --digit) {
       __syncthreads();
-      for (int i = t; i < 256; i += blockDim.x) hist[i] = 0;
+      s_digit[t] = 0;
       __syncthreads();
-      for (int j = t; j < len; j += blockDim.x) {
+      auto add = [&](unsigned long long k) {
+        if ((k & mask) == prefix) atomicAdd(&s_digit[(k >> (8 * digit)) & 255ull], 1);
+      };
+      if (held)
+        for (int j = t; j < q.count; j += blockDim.x) add(sm.keys[c * room + j]);
+      for (int j = t; !held && j < len; j += blockDim.x) {
         const int i = sphere(j);
         float yz, xl, xh;
         if (yz_step(i, yz) > limit) continue;
         x_ends(i, xl, xh);
-        if (abs(step_in(c, yz, xl, xh) - q.step) > 1) continue;
-        const unsigned long long k = key_of(i, c);
-        if ((k & mask) == prefix) atomicAdd(&hist[(k >> (8 * digit)) & 255ull], 1);
+        if (abs(step_in(c, yz, xl, xh) - q.step) <= 1) add(key_of(i, c));
       }
       __syncthreads();
-      int b = 0;
-      while (b < 255 && hist[b] < rank) rank -= hist[b++];
+      int before;
+      const int b = reach(s_digit, 256, rank, before);
+      rank -= before;
       prefix |= static_cast<unsigned long long>(b) << (8 * digit);
       mask |= 255ull << (8 * digit);
     }
