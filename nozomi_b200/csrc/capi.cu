@@ -64,6 +64,21 @@ static int check_substrate(const nz_substrate* s, const char* who) {
   return NZ_OK;
 }
 
+// Whether the plain step takes several lanes a walker over the index lists,
+// or one over the spheres' arrays: by the mean entries a cell.  The lanes of a
+// walker each draw its jumps, which short lists do not repay once the walkers
+// fill the GPU by themselves.  Microseconds a step, arrays / lists, without
+// directions: 0 entries 1e6 walkers 23 / 76; 1.6 entries 5.5e4 26.8 / 25.1,
+// 2.5e5 37 / 44; 3.1 entries 2.5e5 54.6 / 53.6, 1e6 124 / 156; 5.6 entries 1e6
+// 209 / 203; 11 entries 1e6 403 / 280.  With directions few walkers gain from
+// the lists' form at any length, as its phases are written by whole lines:
+// 5,000 walkers x 30 take 15.5 / 11.0 at 0.1 entries.
+static bool plain_by_lists(const nz_substrate& sub, int N, int mode, int ndir, long long ncell) {
+  if (sub.S > 0 && sub.n_items <= 0) return true;  // length not given
+  if (N <= 16384 && (mode & NZ_MODE_PHASE) && ndir >= 8) return true;
+  return double(sub.n_items) >= min(6.0, max(1.5, 1.2e-5 * N)) * double(ncell);
+}
+
 extern "C" int nz_walk_step(const nz_substrate* sub, const nz_walkers* wk, int mode, float dt, float G, float Garea,
                             int step, const nz_draws* draws, void* stream) {
   int rc = check_substrate(sub, "nz_walk_step");
@@ -112,7 +127,8 @@ extern "C" int nz_walk_step(const nz_substrate* sub, const nz_walkers* wk, int m
   // index lists, where the substrate has them, hold the same members
   const int width = sub->idx_bytes & ~NZ_NEAR_PACKED;
   if ((width == 2 || width == 4) && sub->cell_idx && sub->rec4 && sub->rec_sid && sub->sid_start &&
-      aligned16(sub->rec4) && (width == 4 || sub->S <= 65536))
+      aligned16(sub->rec4) && (width == 4 || sub->S <= 65536) &&
+      plain_by_lists(*sub, wk->N, mode, wk->ndir, a.ncell))
     return launch_plain_lists(a,
                               PlainLists{sub->cell_idx, reinterpret_cast<const float4*>(sub->rec4), sub->rec_sid,
                                          sub->sid_start},
