@@ -78,6 +78,7 @@ constexpr int kModeDisp = 32;
 struct JobDev {
   Grid g;
   float idLx, idLy, idLz;  // 1 / cell edge (the fused walk's per-step cell)
+  int nx, ny;              // g.nLx, g.nLy
   int nstructures;
   const float4* sph4;
   const int* sid;

@@ -226,6 +226,23 @@ __device__ __forceinline__ uint32_t near_bits_packed(const uint4* __restrict__ p
   return bits;
 }
 
+// The marked entries that a jump below kTinyJump2 can come near, out of line.
+template <int LK, bool SH>
+__device__ __noinline__ uint32_t close_bits(uint32_t bits, const void* __restrict__ list,
+                                            const float4* __restrict__ rec, int first, float x, float y, float z,
+                                            float a, float jr, int S, int& oob) {
+  uint32_t keep = 0u;
+  while (bits) {
+    const int bit = __ffs(bits) - 1;
+    bits &= bits - 1u;
+    int key;
+    float4 c;
+    entry<LK, SH>(list, rec, nullptr, first + bit_entry(bit), S, oob, key, c);
+    if (!beyond(x - c.x, y - c.y, z - c.z, c.w, a, jr)) keep |= 1u << bit;
+  }
+  return keep;
+}
+
 // Fractions of the marked entries of one walker (bits, as near_bits marks
 // them, of the entries from list position `first` on): the reference's inside
 // test, then the fraction of a containing sphere or of a lower structure's
@@ -235,8 +252,7 @@ template <int LK, bool T64, bool SH>
 __device__ __forceinline__ void fractions(uint32_t bits, const void* __restrict__ list,
                                           const float4* __restrict__ rec, const int* __restrict__ sid, int first,
                                           int lo, int hi, float x, float y, float z, float a, float jx, float jy,
-                                          float jz, float jr, int S, int& oob, ScanOut& o, bool& lower,
-                                          int& within) {
+                                          float jz, int S, int& oob, ScanOut& o, bool& lower, int& within) {
   while (bits) {
     const int i = bit_entry(__ffs(bits) - 1);
     bits &= bits - 1u;
@@ -246,7 +262,6 @@ __device__ __forceinline__ void fractions(uint32_t bits, const void* __restrict_
     if (key >= hi) continue;
     const bool below = key < lo;
     const float dx = x - c.x, dy = y - c.y, dz = z - c.z;
-    if (beyond(dx, dy, dz, c.w, a, jr)) continue;
     const float d2 = dx * dx + dy * dy + dz * dz;
     const bool inside = d2 - c.w * c.w < 0;
     if (inside || below) {
@@ -398,7 +413,7 @@ __device__ __forceinline__ int step_cell(const JobDev& J, float x, float y, floa
   mx = __fmaf_rn(cx, g.dLx, 0.5f * (g.dLx - g.Lx));
   my = __fmaf_rn(cy, g.dLy, 0.5f * (g.dLy - g.Ly));
   mz = __fmaf_rn(cz, g.dLz, 0.5f * (g.dLz - g.Lz));
-  return cell_index(g, cx, cy, cz);
+  return cell_index(J.nx, J.ny, cx, cy, cz);
 }
 
 // Start and count of cell `cell`'s list (the near list when near).  In the
@@ -545,7 +560,7 @@ __device__ __forceinline__ void walk_warp(const JobDev& J, bool live, int w, int
     bool lower = false;
     bool more = act && !deep && count > 0;
     const bool packed = LK != 0 && J.near_pack != nullptr;
-    const bool tiny = a < kTinyJump2;  // every entry is marked; fractions passes over the far ones
+    const bool tiny = a < kTinyJump2;  // every entry is marked; close_bits passes over the far ones
     const float inf = __int_as_float(0x7f800000);
     const void* list = LK ? (near ? J.near_idx : J.idx) : nullptr;
     const float4* rec = LK ? J.rec4 : (near ? J.near_sph4 : J.sph4);
@@ -615,9 +630,10 @@ __device__ __forceinline__ void walk_warp(const JobDev& J, bool live, int w, int
           oob |= bad;
         }
       }
+      if (tiny && bits) bits = close_bits<LK, SH>(bits, list, rec, start + base, x, y, z, a, jr, J.S, oob);
       if (bits)
-        fractions<LK, kT64, SH>(bits, list, rec, sid, start + base, lo, hi, x, y, z, a, jx, jy, jz, jr, J.S, oob, r,
-                                lower, within);
+        fractions<LK, kT64, SH>(bits, list, rec, sid, start + base, lo, hi, x, y, z, a, jx, jy, jz, J.S, oob, r, lower,
+                                within);
       more = more && base + 32 < count;
     }
     if (!act) continue;
@@ -1216,6 +1232,8 @@ __host__ __device__ JobDev make_job(const nz_substrate& sub, const float* G, con
   j.idLx = 1.0f / sub.grid.dLx;
   j.idLy = 1.0f / sub.grid.dLy;
   j.idLz = 1.0f / sub.grid.dLz;
+  j.nx = sub.grid.nx;
+  j.ny = sub.grid.ny;
   j.nstructures = sub.nstructures;
   j.ncell = sub.grid.nx * sub.grid.ny * sub.grid.nz;
   j.sph4 = reinterpret_cast<const float4*>(sub.cell_sph4);
