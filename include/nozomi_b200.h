@@ -45,6 +45,7 @@ extern "C" {
  * per-entry record lists) */
 #define NZ_LIST_IDX16 64    /* substrates with idx_bytes 2 */
 #define NZ_LIST_IDX32 128   /* substrates with idx_bytes 4 */
+#define NZ_LIST_PACKED 512  /* with either: substrates whose idx_bytes carry NZ_NEAR_PACKED */
 
 /* added to nz_substrate.idx_bytes: near_sph4 holds packed near entries (nz_cells_pack) */
 #define NZ_NEAR_PACKED 256
@@ -364,7 +365,9 @@ int nz_walk_fused_moments(const nz_substrate* sub, const nz_state* st, int mode,
  * 32 up to 256); an item holds at most `threads` walkers.  The batched form of
  * the fused walk: many substrates, protocols and walker sets in one launch.
  * mode may carry NZ_LIST_IDX16 or NZ_LIST_IDX32: every job's substrate then
- * has index lists of that width (otherwise every job's has record lists).
+ * has index lists of that width (otherwise every job's has record lists), and
+ * with either NZ_LIST_PACKED: the near lists of every job's are packed
+ * (without it packed entries are not read; the results are the same).
  * The device arrays are not read back for checking: the caller guarantees
  * 0 <= item.job < n_jobs, 1 <= item.count <= threads,
  * item.first + item.count <= that job's state.N, and the list format. */

@@ -20,6 +20,7 @@ LIB_PATH = Path(__file__).resolve().parent / ("libnozomi_b200_debug.so" if DEBUG
 NZ_OK, NZ_ERR_ARG, NZ_ERR_CUDA, NZ_ERR_CAPACITY, NZ_ERR_UNSEEDED = 0, 1, 2, 3, 4
 MODE_SIG, MODE_PHASE, MODE_PHI, MODE_MOMENTS, MODE_TANGENT64 = 1, 2, 4, 8, 16
 LIST_IDX16, LIST_IDX32 = 64, 128  # nz_walk_batch: the jobs' list format (none: per-entry records)
+LIST_PACKED = 512  # with either: every job's near lists are packed
 NEAR_PACKED = 256  # added to Substrate.idx_bytes: near_sph4 holds packed near entries (nz_cells_pack)
 FLAG_DRAWS_EXHAUSTED, FLAG_ITER_CAP, FLAG_UNSEEDED, FLAG_BOUNDS, FLAG_STAGE_TIMEOUT = 1, 2, 4, 8, 16
 MAX_STAGE_RECORDS = 12288  # nz_walk_batch_staged: records a CTA stages in shared memory at most

@@ -139,6 +139,16 @@ def _sort_table(pairs, coarsen, by_label):
 LIST_BITS = {0: 0, 2: L.LIST_IDX16, 4: L.LIST_IDX32}
 
 
+def _mode(lk: int, packed: bool) -> int:
+    return L.MODE_PHI | LIST_BITS[lk] | (L.LIST_PACKED if lk and packed else 0)
+
+
+def all_packed(subs) -> bool:
+    """Whether the near lists of all these substrates are packed: the batched
+    walk then takes them."""
+    return all(s.near_packed for s in subs)
+
+
 def list_groups(jobs, active) -> dict:
     """Active jobs by the list form of their substrate (idx_bytes): one
     batched launch per form."""
@@ -148,30 +158,32 @@ def list_groups(jobs, active) -> dict:
     return groups
 
 
-def batch_grid(threads: int, lk: int, stage: int = 0) -> int:
+def batch_grid(threads: int, lk: int, stage: int = 0, packed: bool = False) -> int:
     """Persistent grid of the batched walk: CTAs resident per SM x SMs
-    (with `stage` records of shared memory per CTA for index lists)."""
+    (with `stage` records of shared memory per CTA for index lists; packed:
+    over packed near lists)."""
     dev = torch.device("cuda", torch.cuda.current_device())
     sms = torch.cuda.get_device_properties(dev).multi_processor_count
     occ = ctypes.c_int(0)
     lib = L.load()
     if stage and lk:
-        L.check(lib.nz_batch_occupancy_staged(L.MODE_PHI | LIST_BITS[lk], int(threads), int(stage),
+        L.check(lib.nz_batch_occupancy_staged(_mode(lk, packed), int(threads), int(stage),
                                               ctypes.byref(occ)), "nz_batch_occupancy_staged")
     else:
-        L.check(lib.nz_batch_occupancy(L.MODE_PHI | LIST_BITS[lk], int(threads), ctypes.byref(occ)),
+        L.check(lib.nz_batch_occupancy(_mode(lk, packed), int(threads), ctypes.byref(occ)),
                 "nz_batch_occupancy")
     return sms * max(1, occ.value)
 
 
 def launch_batch(table, n_jobs: int, items, lk: int, s0: int, s1: int, queue_ptr: int, grid: int, threads: int,
-                 stage: int, stream) -> None:
+                 stage: int, stream, packed: bool = False) -> None:
     """One batched walk launch over `items` (list form lk): nz_walk_batch, or
     nz_walk_batch_staged when `stage` records per CTA are staged (index lists
-    only; record lists are never staged)."""
+    only; record lists are never staged).  packed: the near lists of every
+    item's substrate are packed."""
     lib = L.load()
     args = (ctypes.c_void_p(table.data_ptr()), int(n_jobs), ctypes.c_void_p(items.data_ptr()), int(items.shape[0]),
-            L.MODE_PHI | LIST_BITS[lk], int(s0), int(s1), ctypes.c_void_p(queue_ptr), int(grid), int(threads))
+            _mode(lk, packed), int(s0), int(s1), ctypes.c_void_p(queue_ptr), int(grid), int(threads))
     if stage and lk:
         L.check(lib.nz_walk_batch_staged(*args, int(stage), stream), "nz_walk_batch_staged")
     else:
@@ -231,8 +243,9 @@ class BatchRun:
         # and amplitudes above, plus positions given as host arrays and the
         # chunk tables (added by prepare)
         self.h2d_bytes = sum(j["G"].numel() * 8 + j["dirs"].numel() * 4 + j["amps"].numel() * 4 for j in self.jobs)
-        self.grids = {lk: batch_grid(self.threads, lk, self.tuning.stage)
-                      for lk in {j["sub"].idx_bytes for j in self.jobs}}
+        forms = {j["sub"].idx_bytes for j in self.jobs}
+        self.packed = {lk: all_packed(j["sub"] for j in self.jobs if j["sub"].idx_bytes == lk) for lk in forms}
+        self.grids = {lk: batch_grid(self.threads, lk, self.tuning.stage, self.packed[lk]) for lk in forms}
         self.grid = max(self.grids.values())
         self._planned = False
 
@@ -326,7 +339,7 @@ class BatchRun:
             for g, (lk, items) in enumerate(c["launches"]):
                 launch_batch(c["table"], len(self.jobs), items, lk, c["s0"], c["s1"],
                              self.queue.data_ptr() + 4 * (3 * qi + g), self.grids[lk], self.threads,
-                             self.tuning.stage, stream)
+                             self.tuning.stage, stream, self.packed[lk])
             if events is not None:
                 e1.record(cs)
                 events.append((e0, e1))

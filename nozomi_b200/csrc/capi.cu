@@ -212,7 +212,9 @@ static int check_fused_sub(const nz_substrate* sub, const char* who) {
 
 // List kind of an nz_walk_batch launch from its mode bits.
 static int batch_list_kind(int mode) {
-  if ((mode & NZ_LIST_IDX16) && (mode & NZ_LIST_IDX32)) return -1;
+  const int lists = mode & (NZ_LIST_IDX16 | NZ_LIST_IDX32 | NZ_LIST_PACKED);
+  if ((lists & NZ_LIST_IDX16) && (lists & NZ_LIST_IDX32)) return -1;
+  if (lists == NZ_LIST_PACKED) return -1;
   return (mode & NZ_LIST_IDX16) ? 2 : (mode & NZ_LIST_IDX32) ? 4 : 0;
 }
 
@@ -300,14 +302,14 @@ static int walk_batch(const char* what, const nz_job* jobs, int n_jobs, const nz
   if (grid > 0 && !queue) return set_error(NZ_ERR_ARG, "%s: a persistent grid needs a queue counter", what);
   if (mode & NZ_MODE_MOMENTS) return set_error(NZ_ERR_ARG, "%s: moments are per-substrate (nz_walk_fused)", what);
   const int lk = batch_list_kind(mode);
-  if (lk < 0) return set_error(NZ_ERR_ARG, "%s: both list widths in mode %d", what, mode);
+  if (lk < 0) return set_error(NZ_ERR_ARG, "%s: both list widths or packed lists of none in mode %d", what, mode);
   if (stage_records < 0 || stage_records > kMaxStageRecords)
     return set_error(NZ_ERR_ARG, "%s: stage_records %d outside [0, %d]", what, stage_records, kMaxStageRecords);
   if (stage_records > 0 && lk == 0)
     return set_error(NZ_ERR_ARG, "%s: records are staged for index lists only (no NZ_LIST_IDX bit in mode)", what);
   if (n_items == 0 || step1 == step0) return NZ_OK;
   const JobDev unused{};
-  return launch_fused(mode & ~(NZ_LIST_IDX16 | NZ_LIST_IDX32), lk, unused, jobs, items, n_items, step0, step1,
+  return launch_fused(mode, lk, unused, jobs, items, n_items, step0, step1,
                       grid > 0 ? queue : nullptr, grid > 0 ? grid : n_items, threads,
                       static_cast<cudaStream_t>(stream), stage_records);
 }
@@ -329,7 +331,7 @@ extern "C" int nz_batch_occupancy(int mode, int threads, int* blocks_per_sm) {
   const int lk = batch_list_kind(mode);
   if (!blocks_per_sm || threads < 32 || threads > kFusedMaxThreads || lk < 0)
     return set_error(NZ_ERR_ARG, "nz_batch_occupancy: bad arguments");
-  return occupancy_fused(mode & ~(NZ_LIST_IDX16 | NZ_LIST_IDX32), lk, threads, blocks_per_sm);
+  return occupancy_fused(mode, lk, threads, blocks_per_sm);
 }
 
 extern "C" int nz_batch_occupancy_staged(int mode, int threads, int stage_records, int* blocks_per_sm) {
@@ -337,5 +339,5 @@ extern "C" int nz_batch_occupancy_staged(int mode, int threads, int stage_record
   if (!blocks_per_sm || threads < 32 || threads > kFusedMaxThreads || lk <= 0 || stage_records < 0 ||
       stage_records > kMaxStageRecords)
     return set_error(NZ_ERR_ARG, "nz_batch_occupancy_staged: bad arguments");
-  return occupancy_fused(mode & ~(NZ_LIST_IDX16 | NZ_LIST_IDX32), lk, threads, blocks_per_sm, stage_records);
+  return occupancy_fused(mode, lk, threads, blocks_per_sm, stage_records);
 }

@@ -119,16 +119,15 @@ __device__ __forceinline__ bool beyond(float dx, float dy, float dz, float r, fl
 // iteration whose label had to be corrected.
 template <int LK, bool T64, bool SH>
 __device__ __noinline__ void scan_lane(const void* __restrict__ list, const float4* __restrict__ rec,
-                                          const int* __restrict__ sid, int start, int count, int lo, int hi, float x,
-                                          float y, float z, float a, float jx, float jy, float jz, float jr, int S,
-                                          int& oob, ScanOut& o) {
+                                       int start, int count, int lo, int hi, float x, float y, float z, float a,
+                                       float jx, float jy, float jz, float jr, int S, int& oob, ScanOut& o) {
   o.fin = 0.0f;
   o.fout = kBig;
   o.any_in = false;
   for (int i = 0; i < count; ++i) {
     int key;
     float4 c;
-    entry<LK, SH>(list, rec, sid, start + i, S, oob, key, c);
+    entry<LK, SH>(list, rec, nullptr, start + i, S, oob, key, c);
     if (key >= hi) break;
     const float dx = x - c.x, dy = y - c.y, dz = z - c.z;
     if (beyond(dx, dy, dz, c.w, a, jr)) continue;
@@ -171,33 +170,7 @@ __device__ __forceinline__ bool is_near(const Reach& g, float x, float y, float 
 // Near masks cover 32 list entries: entry i at bit (i >> 1) | (i & 1) << 4.
 __device__ __forceinline__ int bit_entry(int bit) { return 2 * (bit & 15) + (bit >> 4); }
 
-// Near mask of `n` (at most 32) entries from list position `first` on, from
-// their records; entries of a structure above the walker's are left out (keys
-// ascend).
-template <int LK, bool SH>
-__device__ __forceinline__ uint32_t near_bits(const void* __restrict__ list, const float4* __restrict__ rec,
-                                              const int* __restrict__ sid, int first, int n, int hi, int S, int& oob,
-                                              const Reach& g, float x, float y, float z) {
-  uint32_t bits = 0u;
-  bool stop = false;
-  // four entries at a time, their loads (two dependent ones each) in flight
-  // together
-  for (int i0 = 0; i0 < n && !stop; i0 += 4) {
-    int key[4];
-    float4 c[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) entry<LK, SH>(list, rec, sid, first + min(i0 + u, n - 1), S, oob, key[u], c[u]);
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const bool valid = key[u] < hi && i0 + u < n;
-      stop |= key[u] >= hi;
-      bits |= valid && is_near(g, x, y, z, c[u]) ? 1u << ((i0 >> 1) + (u >> 1) + 16 * (u & 1)) : 0u;
-    }
-  }
-  return bits;
-}
-
-// The same for the packed near entries (nz_cells_pack) of up to 16 pairs, two
+// Near mask of up to 16 pairs of packed near entries (nz_cells_pack), two
 // entries an instruction in half precision: px.. the position relative to
 // the cell's centre, ex.. the segment's direction, len its length, grow 2 %
 // of it.  The entries' radii hold the rounding of these distances.
@@ -250,15 +223,15 @@ __device__ __noinline__ uint32_t close_bits(uint32_t bits, const void* __restric
 // a sphere of a lower structure contains the walker.
 template <int LK, bool T64, bool SH>
 __device__ __forceinline__ void fractions(uint32_t bits, const void* __restrict__ list,
-                                          const float4* __restrict__ rec, const int* __restrict__ sid, int first,
-                                          int lo, int hi, float x, float y, float z, float a, float jx, float jy,
-                                          float jz, int S, int& oob, ScanOut& o, bool& lower, int& within) {
+                                          const float4* __restrict__ rec, int first, int lo, int hi, float x, float y,
+                                          float z, float a, float jx, float jy, float jz, int S, int& oob, ScanOut& o,
+                                          bool& lower, int& within) {
   while (bits) {
     const int i = bit_entry(__ffs(bits) - 1);
     bits &= bits - 1u;
     int key;
     float4 c;
-    entry<LK, SH>(list, rec, sid, first + i, S, oob, key, c);
+    entry<LK, SH>(list, rec, nullptr, first + i, S, oob, key, c);
     if (key >= hi) continue;
     const bool below = key < lo;
     const float dx = x - c.x, dy = y - c.y, dz = z - c.z;
@@ -269,7 +242,7 @@ __device__ __forceinline__ void fractions(uint32_t bits, const void* __restrict_
       const float f = T64 ? step_either_t<T64>(inside, dx, dy, dz, c.w, a, jx, jy, jz)
                           : step_one(inside, dx, dy, dz, d2, c.w, a, jx, jy, jz);
       if (inside) {
-        if (LK != 0 && (!o.any_in || o.fin < f)) within = key;
+        if (!o.any_in || o.fin < f) within = key;
         o.any_in = true;
         if (o.fin < f) o.fin = f;
       } else if (f < o.fout) {
@@ -461,6 +434,7 @@ __device__ __forceinline__ void jump_of(const JobDev& J, uint32_t wid, int s, in
 template <int MODE, int LK, bool SH>
 __device__ __forceinline__ void walk_warp(const JobDev& J, bool live, int w, int s0, int s1,
                                           double* s_mom, float4* s_phi) {
+  static_assert(LK != 0, "index lists only");
   constexpr bool kMom = (MODE & NZ_MODE_MOMENTS) != 0;
   constexpr bool kDisp = (MODE & kModeDisp) != 0;
   constexpr bool kOrig = kMom || kDisp;  // origin in registers
@@ -491,7 +465,7 @@ __device__ __forceinline__ void walk_warp(const JobDev& J, bool live, int w, int
   int lo = 0, hi = 0;  // keys of structure `label`
   int within = -1;     // index form: record of a sphere that contained the walker (-1: none known)
   const float dt = J.dt;
-  const bool has_near = (LK ? J.near_idx : static_cast<const void*>(J.near_sph4)) != nullptr;
+  const bool has_near = J.near_pack != nullptr;  // else the warp tests the full lists
   if (live) {
     const float4 P = J.pos[w];
     x = P.x; y = P.y; z = P.z;
@@ -539,35 +513,30 @@ __device__ __forceinline__ void walk_warp(const JobDev& J, bool live, int w, int
     // sphere that held the walker longest when its fractions were last
     // computed.
     bool deep = false;
-    if (LK != 0 && J.rec_safe && within >= lo && within < hi && near && a >= kTinyJump2) {
+    if (within >= lo && within < hi && near && a >= kTinyJump2) {
       const float4 c = SH ? s_stage[within] : __ldg(J.rec4 + within);
       const float safe = __ldg(J.rec_safe + within);
       const float dx = x - c.x, dy = y - c.y, dz = z - c.z;
       const float ux = __fmaf_rn(jr, jx, dx), uy = __fmaf_rn(jr, jy, dy), uz = __fmaf_rn(jr, jz, dz);
       deep = fmaxf(__fmaf_rn(dx, dx, __fmaf_rn(dy, dy, dz * dz)), __fmaf_rn(ux, ux, __fmaf_rn(uy, uy, uz * uz))) < safe;
     }
-    // The collision pass.  Each lane marks its list's near entries 32 at a
-    // time and computes their fractions:
-    //  * packed near lists (the usual case): near_bits_packed;
-    //  * an iteration that needs the full list where near lists are packed (1
-    //    walker in 100): the warp tests that list together, an entry a lane,
-    //    so the others do not wait for a lane's 20 and more entries;
-    //  * lists without packed entries: near_bits.
+    // The collision pass.  Each lane marks its near list's near entries 32 at
+    // a time (near_bits_packed) and computes their fractions.  Where an
+    // iteration needs the full list (1 walker in 100) the warp tests that list
+    // together, an entry a lane, so the others do not wait for a lane's 20 and
+    // more entries.
     ScanOut r;
     r.fin = 0.0f;
     r.fout = kBig;
     r.any_in = false;
     bool lower = false;
     bool more = act && !deep && count > 0;
-    const bool packed = LK != 0 && J.near_pack != nullptr;
     const bool tiny = a < kTinyJump2;  // every entry is marked; close_bits passes over the far ones
     const float inf = __int_as_float(0x7f800000);
-    const void* list = LK ? (near ? J.near_idx : J.idx) : nullptr;
-    const float4* rec = LK ? J.rec4 : (near ? J.near_sph4 : J.sph4);
-    const int* sid = LK ? nullptr : (near ? J.near_sid : J.sid);
-    const unsigned full0 = packed ? __ballot_sync(kAll, more && !near) : 0u;
+    const void* list = near ? J.near_idx : J.idx;
+    const unsigned full0 = __ballot_sync(kAll, more && !near);
     Reach g;
-    if (!packed || full0) {
+    if (full0) {
       const float f = 2.0f * jr;
       g.mx = f * jx;
       g.my = f * jy;
@@ -576,29 +545,17 @@ __device__ __forceinline__ void walk_warp(const JobDev& J, bool live, int w, int
       g.k = -0.5f * rcp_approx(g.m2);
       g.slack = tiny ? inf : kTol + 2e-3f + 0.02f * reach;
     }
-    __half2 px, py, pz, ex, ey, ez, len, grow;
-    const uint4* pk = nullptr;
-    if (packed) {
-      const float ir = rsqrt_approx(fmaxf(a, 1e-30f));
-      px = __float2half2_rn(x - mx);
-      py = __float2half2_rn(y - my);
-      pz = __float2half2_rn(z - mz);
-      ex = __float2half2_rn(jx * ir);
-      ey = __float2half2_rn(jy * ir);
-      ez = __float2half2_rn(jz * ir);
-      len = __float2half2_rn(reach);
-      grow = __float2half2_rn(tiny ? inf : 0.02f * reach);
-      pk = J.near_pack + ((start + cell + 1) >> 1);
-    }
+    const float ir = rsqrt_approx(fmaxf(a, 1e-30f));
+    const __half2 px = __float2half2_rn(x - mx), py = __float2half2_rn(y - my), pz = __float2half2_rn(z - mz);
+    const __half2 ex = __float2half2_rn(jx * ir), ey = __float2half2_rn(jy * ir), ez = __float2half2_rn(jz * ir);
+    const __half2 len = __float2half2_rn(reach), grow = __float2half2_rn(tiny ? inf : 0.02f * reach);
+    const uint4* pk = J.near_pack + ((start + cell + 1) >> 1);
     for (int base = 0; __any_sync(kAll, more); base += 32) {
       uint32_t bits = 0u;
-      if (more) {
+      if (more && near) {
         const int n = min(32, count - base);
-        if (!packed)
-          bits = near_bits<LK, SH>(list, rec, sid, start + base, n, hi, J.S, oob, g, x, y, z);
-        else if (near)
-          bits = near_bits_packed(pk + (base >> 1), (n + 1) >> 1, px, py, pz, ex, ey, ez, len, grow) &
-                 (((1u << ((n + 1) >> 1)) - 1u) | (((1u << (n >> 1)) - 1u) << 16));
+        bits = near_bits_packed(pk + (base >> 1), (n + 1) >> 1, px, py, pz, ex, ey, ez, len, grow) &
+               (((1u << ((n + 1) >> 1)) - 1u) | (((1u << (n >> 1)) - 1u) << 16));
       }
       unsigned full = full0 ? __ballot_sync(kAll, more && !near) : 0u;
       while (full) {
@@ -630,10 +587,9 @@ __device__ __forceinline__ void walk_warp(const JobDev& J, bool live, int w, int
           oob |= bad;
         }
       }
-      if (tiny && bits) bits = close_bits<LK, SH>(bits, list, rec, start + base, x, y, z, a, jr, J.S, oob);
+      if (tiny && bits) bits = close_bits<LK, SH>(bits, list, J.rec4, start + base, x, y, z, a, jr, J.S, oob);
       if (bits)
-        fractions<LK, kT64, SH>(bits, list, rec, sid, start + base, lo, hi, x, y, z, a, jx, jy, jz, J.S, oob, r, lower,
-                                within);
+        fractions<LK, kT64, SH>(bits, list, J.rec4, start + base, lo, hi, x, y, z, a, jx, jy, jz, J.S, oob, r, lower, within);
       more = more && base + 32 < count;
     }
     if (!act) continue;
@@ -645,7 +601,7 @@ __device__ __forceinline__ void walk_warp(const JobDev& J, bool live, int w, int
     // the label carried from the previous iteration holds when no sphere of a
     // lower structure contains the walker and, outside the box, one of its own does
     if (lower || (label < J.nstructures && !r.any_in)) {
-      label = label_of<LK, SH>(list, rec, sid, J.rec_sid, start, count, J.nstructures, x, y, z, J.S, oob);
+      label = label_of<LK, SH>(list, J.rec4, nullptr, J.rec_sid, start, count, J.nstructures, x, y, z, J.S, oob);
       if (kCheckBounds && (label < 0 || label > J.nstructures)) {
         oob = 1;
         label = J.nstructures;
@@ -660,8 +616,7 @@ __device__ __forceinline__ void walk_warp(const JobDev& J, bool live, int w, int
       // the full list: the near one was chosen for the old reach
       int fs, fc;
       cell_list(J, false, cell, fs, fc, oob);
-      scan_lane<LK, kT64, SH>(LK ? J.idx : nullptr, LK ? J.rec4 : J.sph4, LK ? nullptr : J.sid, fs, fc, lo, hi, x, y,
-                              z, a, jx, jy, jz, jr, J.S, oob, r);
+      scan_lane<LK, kT64, SH>(J.idx, J.rec4, fs, fc, lo, hi, x, y, z, a, jx, jy, jz, jr, J.S, oob, r);
     }
     jc = ref_min(jc, r.any_in ? r.fin : kBig);
     jc = ref_min(jc, r.fout);
@@ -1066,13 +1021,15 @@ __device__ __forceinline__ void stage_records(uint32_t bar, const float4* src, u
 #else
 #define NZ_FUSED_BOUNDS __launch_bounds__(kFusedMaxThreads, kFusedMinBlocks)
 #endif
-enum : int { kBatch, kSingle, kSinglePacked };  // kinds of launch: one job with or without packed near lists
+// kinds of launch: many jobs or one, their near lists packed (walk_warp) or not (walk_one)
+enum : int { kBatch, kBatchPacked, kSingle, kSinglePacked };
 template <int MODE, int LK, int KIND, bool STAGE>
 __global__ void NZ_FUSED_BOUNDS
     walk_fused_kernel(const __grid_constant__ JobDev single, const nz_job* __restrict__ jobs,
                       const nz_item* __restrict__ items, int n_items, int step0, int step1, int* queue,
                       int stage_cap) {
-  constexpr bool SINGLE = KIND != kBatch;
+  constexpr bool SINGLE = KIND == kSingle || KIND == kSinglePacked;
+  constexpr bool PACKED = KIND == kBatchPacked || KIND == kSinglePacked;
   static_assert(!STAGE || (!SINGLE && LK != 0), "staging is for batched index-list walks");
   __shared__ int s_item;
   __shared__ double s_mom[(MODE & NZ_MODE_MOMENTS) ? kMomentSteps * 6 : 1];
@@ -1109,7 +1066,7 @@ __global__ void NZ_FUSED_BOUNDS
       const int per = int(blockDim.x >> 5) * lanes;
       const int first = it * per;
       const int count = min(per, single.nwalkers - first);
-      run_item<MODE, LK, false, KIND == kSinglePacked>(single, first, count, step0, step1, s_mom, s_phi, 0, lanes);
+      run_item<MODE, LK, false, PACKED>(single, first, count, step0, step1, s_mom, s_phi, 0, lanes);
     } else {
       // every thread of the CTA works on the same job: its descriptor lives
       // in shared memory, not in each thread's registers
@@ -1157,10 +1114,10 @@ __global__ void NZ_FUSED_BOUNDS
             }
           }
         }
-        if (use) run_item<MODE, LK, true, true>(s_job, wi.first, wi.count, step0, step1, s_mom, s_phi);
-        else run_item<MODE, LK, false, LK != 0>(s_job, wi.first, wi.count, step0, step1, s_mom, s_phi, flags);
+        if (use) run_item<MODE, LK, true, PACKED>(s_job, wi.first, wi.count, step0, step1, s_mom, s_phi);
+        else run_item<MODE, LK, false, false>(s_job, wi.first, wi.count, step0, step1, s_mom, s_phi, flags);
       } else {
-        run_item<MODE, LK, false, LK != 0>(s_job, wi.first, wi.count, step0, step1, s_mom, s_phi);
+        run_item<MODE, LK, false, PACKED>(s_job, wi.first, wi.count, step0, step1, s_mom, s_phi);
       }
       __syncthreads();
     }
@@ -1278,87 +1235,82 @@ __host__ __device__ JobDev make_job(const nz_substrate& sub, const float* G, con
   return j;
 }
 
-// Dynamic shared memory of the staged kernel for stage_cap records, after
-// setting its attributes: the largest allowed size (once per device) and a
-// carveout that leaves room for the CTAs the register budget allows at this
-// CTA size, the rest staying L1.
-// Shared memory carveout (percent) of the unstaged walk: what the CTAs that
-// the register budget allows need (and 1 KB each that the system takes); the
-// rest stays L1, which the lists and records live in.
+// Shared memory carveout (percent) of the unstaged walk over packed lists:
+// what the CTAs that the register budget allows need (and 1 KB each that the
+// system takes); the rest stays L1, which the lists and records live in.
 template <int MODE>
 constexpr int fused_carveout() {
   constexpr size_t need = kFusedMinBlocks * phi_bytes<MODE>(kFusedMaxThreads) + 2 * kFusedMinBlocks * 1400;
   return phi_bytes<MODE>(32) ? int((100 * need + kSmemPerSm - 1) / kSmemPerSm) : 0;
 }
 
-template <int MODE, int LK>
+// Dynamic shared memory of the staged kernel for stage_cap records, after
+// setting its attributes: the largest allowed size (once per device) and a
+// carveout that leaves room for the CTAs the register budget allows at this
+// CTA size, the rest staying L1.
+template <int MODE, int LK, int KIND>
 size_t stage_setup(int stage_cap, int threads) {
-  const size_t bytes = size_t(stage_cap) * 16 + phi_bytes<MODE>(threads);
-  if (LK == 0 || stage_cap <= 0) return 0;
+  auto kernel = walk_fused_kernel<MODE, LK, KIND, true>;
+  const size_t bytes = size_t(stage_cap) * 16 + (KIND == kBatchPacked ? phi_bytes<MODE>(threads) : 0);
   int dev = 0;
   if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < kMaxDevices) {
     static std::once_flag once[kMaxDevices];
-    std::call_once(once[dev], [] {
-      cudaFuncSetAttribute(walk_fused_kernel<MODE, LK, kBatch, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    std::call_once(once[dev], [&] {
+      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            kMaxStageRecords * 16 + int(phi_bytes<MODE>(kFusedMaxThreads)));
     });
   }
   const int ctas = std::max(1, kFusedMinBlocks * kFusedMaxThreads / threads);
   const size_t need = size_t(ctas) * (bytes + 2048);
   const int pct = int(std::min<size_t>(100, (100 * need + kSmemPerSm - 1) / kSmemPerSm));
-  cudaFuncSetAttribute(walk_fused_kernel<MODE, LK, kBatch, true>, cudaFuncAttributePreferredSharedMemoryCarveout, pct);
+  cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, pct);
   return bytes;
 }
 
+// packed: the near lists of all jobs (of the single one) are packed.
 template <int MODE, int LK>
 void launch_mode(const JobDev& single, const nz_job* jobs, const nz_item* items, int n_items, int step0, int step1,
-                 int* queue, int grid, int threads, int stage_cap, cudaStream_t st) {
-  // the kernel keeps little in shared memory: prefer the whole carveout for
-  // L1.  Function attributes belong to a device's context, so this is done
-  // once per device (and once across threads).
+                 int* queue, int grid, int threads, int stage_cap, bool packed, cudaStream_t st) {
+  // walk_one keeps nothing in shared memory: the whole carveout for L1.
+  // Function attributes belong to a device's context, so this is done once
+  // per device (and once across threads).
   int dev = 0;
   if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < kMaxDevices) {
     static std::once_flag once[kMaxDevices];
     std::call_once(once[dev], [] {
-      cudaFuncSetAttribute(walk_fused_kernel<MODE, LK, kBatch, false>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                           LK ? fused_carveout<MODE>() : 0);
-      cudaFuncSetAttribute(walk_fused_kernel<MODE, LK, kSingle, false>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                           0);
-      if constexpr (LK != 0)
-        cudaFuncSetAttribute(walk_fused_kernel<MODE, LK, kSinglePacked, false>,
-                             cudaFuncAttributePreferredSharedMemoryCarveout, fused_carveout<MODE>());
+      auto carve = [](auto kernel, int pct) {
+        cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, pct);
+      };
+      carve(walk_fused_kernel<MODE, LK, kBatch, false>, 0);
+      carve(walk_fused_kernel<MODE, LK, kSingle, false>, 0);
+      if constexpr (LK != 0) {
+        carve(walk_fused_kernel<MODE, LK, kBatchPacked, false>, fused_carveout<MODE>());
+        carve(walk_fused_kernel<MODE, LK, kSinglePacked, false>, fused_carveout<MODE>());
+      }
     });
   }
+  auto run = [&](auto kernel, size_t smem) {
+    kernel<<<grid, threads, smem, st>>>(single, jobs, items, n_items, step0, step1, queue, stage_cap);
+  };
   if constexpr (LK != 0) {
-    if (jobs && stage_cap > 0) {
-      const size_t smem = stage_setup<MODE, LK>(stage_cap, threads);
-      walk_fused_kernel<MODE, LK, kBatch, true>
-          <<<grid, threads, smem, st>>>(single, jobs, items, n_items, step0, step1, queue, stage_cap);
-      return;
-    }
+    const size_t bytes = phi_bytes<MODE>(threads);
+    if (jobs && stage_cap > 0)
+      return packed ? run(walk_fused_kernel<MODE, LK, kBatchPacked, true>,
+                          stage_setup<MODE, LK, kBatchPacked>(stage_cap, threads))
+                    : run(walk_fused_kernel<MODE, LK, kBatch, true>, stage_setup<MODE, LK, kBatch>(stage_cap, threads));
+    if (jobs && packed) return run(walk_fused_kernel<MODE, LK, kBatchPacked, false>, bytes);
+    if (packed) return run(walk_fused_kernel<MODE, LK, kSinglePacked, false>, bytes);
   }
-  const size_t bytes = phi_bytes<MODE>(threads);
-  if (jobs) {
-    walk_fused_kernel<MODE, LK, kBatch, false>
-        <<<grid, threads, LK ? bytes : 0, st>>>(single, jobs, items, n_items, step0, step1, queue, 0);
-    return;
-  }
-  if constexpr (LK != 0) {
-    if (single.near_pack) {
-      walk_fused_kernel<MODE, LK, kSinglePacked, false>
-          <<<grid, threads, bytes, st>>>(single, jobs, items, n_items, step0, step1, queue, stage_cap);
-      return;
-    }
-  }
-  walk_fused_kernel<MODE, LK, kSingle, false>
-      <<<grid, threads, 0, st>>>(single, jobs, items, n_items, step0, step1, queue, stage_cap);
+  if (jobs) run(walk_fused_kernel<MODE, LK, kBatch, false>, 0);
+  else run(walk_fused_kernel<MODE, LK, kSingle, false>, 0);
 }
 
 template <int LK>
 int launch_lk(int mode, const JobDev& single, const nz_job* jobs, const nz_item* items, int n_items, int step0,
               int step1, int* queue, int grid, int threads, int stage_cap, cudaStream_t st) {
+  const bool packed = jobs ? (mode & NZ_LIST_PACKED) != 0 : single.near_pack != nullptr;
 #define NZ_LAUNCH(M) \
-  launch_mode<(M), LK>(single, jobs, items, n_items, step0, step1, queue, grid, threads, stage_cap, st)
+  launch_mode<(M), LK>(single, jobs, items, n_items, step0, step1, queue, grid, threads, stage_cap, packed, st)
   switch (mode & (NZ_MODE_PHI | NZ_MODE_SIG | NZ_MODE_MOMENTS | NZ_MODE_TANGENT64 | kModeDisp)) {
     case NZ_MODE_PHI | NZ_MODE_TANGENT64: NZ_LAUNCH(NZ_MODE_PHI | NZ_MODE_TANGENT64); break;
     case NZ_MODE_PHI | NZ_MODE_SIG | NZ_MODE_TANGENT64: NZ_LAUNCH(NZ_MODE_PHI | NZ_MODE_SIG | NZ_MODE_TANGENT64); break;
@@ -1376,9 +1328,13 @@ int launch_lk(int mode, const JobDev& single, const nz_job* jobs, const nz_item*
   return check_launch("walk_fused_kernel");
 }
 
-// jobs == null: the single job `single` with n_items CTAs of kFusedThreads walkers.
-// stage_cap > 0 (batched index-list walks): stage the records of jobs of at
-// most stage_cap records in shared memory.
+// jobs == null: the single job `single`, stage_cap walkers a warp, n_items CTAs
+// of kFusedThreads threads.  Batched index-list walks: stage_cap > 0 stages the
+// records of jobs of at most that many in shared memory; NZ_LIST_PACKED in
+// mode takes the walk over packed near lists.  Without that bit each lane
+// walks by itself: unpacked index lists of four jobs, 1.5e5 walkers, 400
+// steps, 256 (128) threads a CTA: 7.2 (6.9) ms so, 8.1 (8.0) through walk_warp;
+// with their records staged 8.5 (9.5) and 9.9 (11.8).
 int launch_fused(int mode, int lk, const JobDev& single, const nz_job* jobs, const nz_item* items, int n_items,
                  int step0, int step1, int* queue, int grid, int threads, cudaStream_t st, int stage_cap) {
   switch (lk) {
@@ -1394,24 +1350,27 @@ int launch_fused(int mode, int lk, const JobDev& single, const nz_job* jobs, con
 }
 
 template <int MODE, int LK>
-cudaError_t occupancy_mode(int threads, int stage_cap, int* blocks_per_sm) {
+cudaError_t occupancy_mode(int threads, int stage_cap, bool packed, int* blocks_per_sm) {
+  auto fit = [&](auto kernel, size_t smem) {
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, kernel, threads, smem);
+  };
   if constexpr (LK != 0) {
-    if (stage_cap > 0) {
-      const size_t smem = stage_setup<MODE, LK>(stage_cap, threads);
-      return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, walk_fused_kernel<MODE, LK, kBatch, true>,
-                                                           threads, smem);
-    }
+    if (stage_cap > 0)
+      return packed ? fit(walk_fused_kernel<MODE, LK, kBatchPacked, true>,
+                          stage_setup<MODE, LK, kBatchPacked>(stage_cap, threads))
+                    : fit(walk_fused_kernel<MODE, LK, kBatch, true>, stage_setup<MODE, LK, kBatch>(stage_cap, threads));
+    if (packed) return fit(walk_fused_kernel<MODE, LK, kBatchPacked, false>, phi_bytes<MODE>(threads));
   }
-  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, walk_fused_kernel<MODE, LK, kBatch, false>,
-                                                       threads, LK ? phi_bytes<MODE>(threads) : 0);
+  return fit(walk_fused_kernel<MODE, LK, kBatch, false>, 0);
 }
 
 template <int LK>
 cudaError_t occupancy_lk(int mode, int threads, int stage_cap, int* blocks_per_sm) {
+  const bool packed = (mode & NZ_LIST_PACKED) != 0;
   switch (mode & (NZ_MODE_PHI | NZ_MODE_SIG | NZ_MODE_MOMENTS)) {
-    case NZ_MODE_PHI: return occupancy_mode<NZ_MODE_PHI, LK>(threads, stage_cap, blocks_per_sm);
-    case NZ_MODE_SIG: return occupancy_mode<NZ_MODE_SIG, LK>(threads, stage_cap, blocks_per_sm);
-    case NZ_MODE_PHI | NZ_MODE_SIG: return occupancy_mode<NZ_MODE_PHI | NZ_MODE_SIG, LK>(threads, stage_cap, blocks_per_sm);
+    case NZ_MODE_PHI: return occupancy_mode<NZ_MODE_PHI, LK>(threads, stage_cap, packed, blocks_per_sm);
+    case NZ_MODE_SIG: return occupancy_mode<NZ_MODE_SIG, LK>(threads, stage_cap, packed, blocks_per_sm);
+    case NZ_MODE_PHI | NZ_MODE_SIG: return occupancy_mode<NZ_MODE_PHI | NZ_MODE_SIG, LK>(threads, stage_cap, packed, blocks_per_sm);
     default: return cudaErrorInvalidValue;
   }
 }

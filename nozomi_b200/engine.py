@@ -230,6 +230,11 @@ class DeviceSubstrate:
         self.near_margin = margin
         self.near = (st, ct, it, sph4, sid, None)
 
+    @property
+    def near_packed(self) -> bool:
+        """Whether there are near lists whose entries are packed."""
+        return bool(self.idx_bytes) and self.near is not None and self.near[3] is not None
+
     def _gather(self):
         """The fused walk's form of the member lists: index entries, or
         per-entry records."""
@@ -287,7 +292,7 @@ class DeviceSubstrate:
             s.near_sph4, s.near_sid, s.near_idx = ptr(sph4), ptr(sid), ptr(nidx)
             s.near_items = int(self.near_n)
         if self.idx_bytes:
-            packed = L.NEAR_PACKED if self.near is not None and self.near[3] is not None else 0
+            packed = L.NEAR_PACKED if self.near_packed else 0
             s.idx_bytes, s.cell_idx = self.idx_bytes + packed, self.cell_idx.data_ptr()
             s.rec4, s.rec_sid, s.sid_start = self.rec4.data_ptr(), self.rec_sid.data_ptr(), self.sid_start.data_ptr()
         return s

@@ -56,7 +56,8 @@ import torch
 
 from . import engine
 from . import _lib as L
-from .batch import JobSpec, SubstrateCache, _items, _job_table, _sort_table, batch_grid, launch_batch, list_groups
+from .batch import (JobSpec, SubstrateCache, _items, _job_table, _sort_table, all_packed, batch_grid, launch_batch,
+                    list_groups)
 from .simulate import Tuning
 from .substrates import cell_grid
 from .waveforms import step_tables
@@ -132,7 +133,8 @@ class Server:
         self.dev = dev
         self.compute = torch.cuda.current_stream(dev)
         self.side = torch.cuda.Stream(dev)
-        self.grids = {lk: batch_grid(threads, lk, self.tuning.stage) for lk in (0, 2, 4)}
+        self.grids = {(lk, packed): batch_grid(threads, lk, self.tuning.stage, packed)
+                      for lk in (0, 2, 4) for packed in (False, True)}
         self.queue = torch.zeros(3, dtype=torch.int32, device=dev)
         self.sort_scratch = torch.empty(1, dtype=torch.uint8, device=dev)
         self.clock = time.perf_counter
@@ -273,7 +275,7 @@ class Server:
                 self.sort_scratch = torch.empty(need, dtype=torch.uint8, device=self.dev)
             table = _job_table(jobs, [j["buf"][j["cur"]] for j in jobs])
             plan = self._as_plan(jobs)
-            groups = [(lk, _items(plan, grp, self.threads, 0, k))
+            groups = [(lk, all_packed(jobs[i]["sub"] for i in grp), _items(plan, grp, self.threads, 0, k))
                       for lk, grp in sorted(list_groups(jobs, range(len(jobs))).items())]
             e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
             e0.record(self.compute)
@@ -281,9 +283,9 @@ class Server:
                                       ctypes.c_void_p(self.sort_scratch.data_ptr()), self.sort_scratch.numel(),
                                       stream), "nz_batch_sort")
             self.queue.zero_()
-            for g, (lk, items) in enumerate(groups):
-                launch_batch(table, len(jobs), items, lk, 0, k, self.queue.data_ptr() + 4 * g, self.grids[lk],
-                             self.threads, self.tuning.stage, stream)
+            for g, (lk, packed, items) in enumerate(groups):
+                launch_batch(table, len(jobs), items, lk, 0, k, self.queue.data_ptr() + 4 * g,
+                             self.grids[lk, packed], self.threads, self.tuning.stage, stream, packed)
             e1.record(self.compute)
             finished, ws = [], 0
             for t in self.active:
