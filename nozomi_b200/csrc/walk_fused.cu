@@ -82,12 +82,14 @@ __device__ __forceinline__ float4 record(const float4* __restrict__ rec, int S, 
 // the record index, the record read from the substrate's record array.  The
 // entries of a cell ascend by key.  In either form the entries of structure
 // L have keys in [lo, hi) (label_bounds): key < hi is "structure <= L" and
-// key < lo "structure < L"; for a walker in the box every key is below lo.
+// key < lo "structure < L"; for a walker in the box every key is below lo
+// (box: record lists then need none).
 template <int LK, bool SH>
 __device__ __forceinline__ void entry(const void* __restrict__ list, const float4* __restrict__ rec,
-                                      const int* __restrict__ sid, int k, int S, int& oob, int& key, float4& c) {
+                                      const int* __restrict__ sid, int k, int S, int& oob, int& key, float4& c,
+                                      bool box = false) {
   if constexpr (LK == 0) {
-    key = __ldg(sid + k);
+    key = box ? -1 : __ldg(sid + k);
     c = __ldg(rec + k);
   } else {
     if constexpr (LK == 2) key = int(__ldg(static_cast<const unsigned short*>(list) + k));
@@ -256,7 +258,8 @@ __device__ __forceinline__ void fractions(uint32_t bits, const void* __restrict_
 // list under assumed label L.  Returns false when the
 // walker's label is not L (then nothing in `o` is used).  Ends at the first
 // entry of a structure above L (the reference skips those spheres, :805-806).
-template <int LK, bool T64, bool SH>
+// BOX: walkers in the box read no structure ids.
+template <int LK, bool T64, bool SH, bool BOX>
 __device__ __forceinline__ bool scan_cell(const void* __restrict__ list, const float4* __restrict__ rec,
                                           const int* __restrict__ sid, int start, int count, int nstructures,
                                           int lo, int hi, float x, float y, float z, int L, float a, float jx,
@@ -266,6 +269,7 @@ __device__ __forceinline__ bool scan_cell(const void* __restrict__ list, const f
   o.any_in = false;
   bool found = false, lower = false, stop = false;
   const float slack = kTol + reach * 1.02f + 2e-3f;
+  const bool box = BOX && L >= nstructures;
   constexpr int kUnroll = 4;
   for (int base = 0; base < count && !stop; base += 32) {
     const int m = min(32, count - base);
@@ -284,7 +288,7 @@ __device__ __forceinline__ bool scan_cell(const void* __restrict__ list, const f
 #pragma unroll
       for (int u = 0; u < kUnroll; ++u) {
         if (i0 + u < m) {
-          entry<LK, SH>(list, rec, sid, start + base + i0 + u, S, oob, key[u], c[u]);
+          entry<LK, SH>(list, rec, sid, start + base + i0 + u, S, oob, key[u], c[u], box);
         } else {  // past the chunk: a NaN record, never near, stops nothing
           key[u] = -1;
           c[u] = make_float4(__int_as_float(0x7fc00000), 0.f, 0.f, 0.f);
@@ -309,7 +313,7 @@ __device__ __forceinline__ bool scan_cell(const void* __restrict__ list, const f
       near_mask &= near_mask - 1;
       int key;
       float4 c;
-      entry<LK, SH>(list, rec, sid, start + base + i, S, oob, key, c);
+      entry<LK, SH>(list, rec, sid, start + base + i, S, oob, key, c, box);
       const bool below = key < lo;
       const float dx = x - c.x, dy = y - c.y, dz = z - c.z;
       const float d2 = dx * dx + dy * dy + dz * dz;
@@ -739,7 +743,7 @@ __device__ __forceinline__ void walk_warp(const JobDev& J, bool live, int w, int
 // compensation and the step's jump; the origin (spins0) and the flag word stay
 // in memory and are updated in place on the rare wrap / iteration-cap events
 // (except with moments, which read the origin every step).
-template <int MODE, int LK, bool SH>
+template <int MODE, int LK, bool SH, bool BOX>
 __device__ __forceinline__ void walk_one(const JobDev& J, int w, int s0, int s1, double* s_mom) {
   constexpr bool kMom = (MODE & NZ_MODE_MOMENTS) != 0;
   constexpr bool kDisp = (MODE & kModeDisp) != 0;
@@ -812,8 +816,8 @@ __device__ __forceinline__ void walk_one(const JobDev& J, int w, int s0, int s1,
     if (has_near && !near) cell_list(J, false, cell, start, count, oob);
     ScanOut r;
     constexpr bool kT64 = (MODE & NZ_MODE_TANGENT64) != 0;
-    if (!scan_cell<LK, kT64, SH>(list, sph4, sidv, start, count, J.nstructures, lo, hi, x, y, z, label, a, jx, jy, jz,
-                             reach, J.S, oob, r)) {
+    if (!scan_cell<LK, kT64, SH, BOX>(list, sph4, sidv, start, count, J.nstructures, lo, hi, x, y, z, label, a, jx, jy,
+                                  jz, reach, J.S, oob, r)) {
       label = label_of<LK, SH>(list, sph4, sidv, J.rec_sid, start, count, J.nstructures, x, y, z, J.S, oob);
       if (kCheckBounds && (label < 0 || label > J.nstructures)) {
         oob = 1;
@@ -830,8 +834,8 @@ __device__ __forceinline__ void walk_one(const JobDev& J, int w, int s0, int s1,
       // the full list: the near one was chosen for the old reach
       int fs, fc;
       cell_list(J, false, cell, fs, fc, oob);
-      scan_cell<LK, kT64, SH>(LK ? J.idx : nullptr, LK ? J.rec4 : J.sph4, LK ? nullptr : J.sid, fs, fc, J.nstructures, lo,
-                          hi, x, y, z, label, a, jx, jy, jz, reach, J.S, oob, r);
+      scan_cell<LK, kT64, SH, BOX>(LK ? J.idx : nullptr, LK ? J.rec4 : J.sph4, LK ? nullptr : J.sid, fs, fc,
+                               J.nstructures, lo, hi, x, y, z, label, a, jx, jy, jz, reach, J.S, oob, r);
     }
     jc = ref_min(jc, r.any_in ? r.fin : kBig);
     jc = ref_min(jc, r.fout);
@@ -940,7 +944,7 @@ __device__ __forceinline__ void walk_one(const JobDev& J, int w, int s0, int s1,
 
 // One work item: walkers [first, first + count) of job J, steps [step0, step1)
 // clamped to the job's protocol.
-template <int MODE, int LK, bool SH, bool WARP>
+template <int MODE, int LK, bool SH, bool WARP, bool BOX = false>
 __device__ __forceinline__ void run_item(const JobDev& J, int first, int count, int step0, int step1, double* s_mom,
                                          float4* s_phi, int flags = 0, int lanes = 32) {
   const int s0 = step0 + J.step_offset, s1 = min(step1 + J.step_offset, J.nsteps);
@@ -952,7 +956,7 @@ __device__ __forceinline__ void run_item(const JobDev& J, int first, int count, 
   const bool live = int(threadIdx.x & 31) < lanes && slot < count && s0 < s1;
   if (WARP ? __any_sync(0xffffffffu, live) : live) {
     if constexpr (WARP) walk_warp<MODE, LK, SH>(J, live, first + slot, s0, s1, s_mom, s_phi);
-    else walk_one<MODE, LK, SH>(J, first + slot, s0, s1, s_mom);
+    else walk_one<MODE, LK, SH, BOX>(J, first + slot, s0, s1, s_mom);
     if (live && flags) {
       float4* c = J.comp + first + slot;
       c->w = __int_as_float(__float_as_int(c->w) | flags);
@@ -1117,7 +1121,13 @@ __global__ void NZ_FUSED_BOUNDS
         if (use) run_item<MODE, LK, true, PACKED>(s_job, wi.first, wi.count, step0, step1, s_mom, s_phi);
         else run_item<MODE, LK, false, false>(s_job, wi.first, wi.count, step0, step1, s_mom, s_phi, flags);
       } else {
-        run_item<MODE, LK, false, PACKED>(s_job, wi.first, wi.count, step0, step1, s_mom, s_phi);
+        // Record lists: walkers in the box need no structure ids.  Leaving them
+        // unread pays for full lists (four jobs, 1.5e5 walkers, 400 steps: 7.9
+        // against 8.5 ms), costs a little for near lists (5.9, 5.7).
+        if (LK == 0 && !s_job.near_sph4)
+          run_item<MODE, LK, false, false, true>(s_job, wi.first, wi.count, step0, step1, s_mom, s_phi);
+        else
+          run_item<MODE, LK, false, PACKED>(s_job, wi.first, wi.count, step0, step1, s_mom, s_phi);
       }
       __syncthreads();
     }

@@ -82,3 +82,16 @@ def test_packed_bit_over_unpacked_lists():
             np.testing.assert_array_equal(getattr(st, k)[o].view(torch.int32).cpu().numpy(), b, err_msg=k)
     occ = ctypes.c_int(0)
     assert L.load().nz_batch_occupancy(L.MODE_PHI | L.LIST_PACKED, 128, ctypes.byref(occ)) != 0
+
+
+def test_record_lists_without_near_lists():
+    """Full record lists, of which walkers in the box read no structure ids."""
+    from nozomi_b200 import simulate
+    specs = _specs()
+    base = simulate.Tuning(steps_per_launch=50, lists="records")
+    _, want = _states(specs, base, 128)
+    for near_free in ((0, 1, 2), (1,)):
+        _, got = _states(specs, base, 128, unpacked=near_free)
+        for g, w in zip(got, want):
+            for a, b in zip(g, w):
+                np.testing.assert_array_equal(a, b)
