@@ -109,7 +109,7 @@ typedef struct nz_substrate {
      * beyond sid_start[L + 1]: no structure id is read per entry. */
     /* idx_bytes may carry NZ_NEAR_PACKED (2 + NZ_NEAR_PACKED or 4 +
      * NZ_NEAR_PACKED): near_sph4 then holds the packed entries of the near
-     * lists (nz_cells_pack, 16-byte aligned; near_items given), which the
+     * lists (nz_cells_pack, 16-byte aligned), which the
      * fused walk's near filter reads instead of the records.  They change how
      * fast entries are passed over, never a result. */
     int idx_bytes;
@@ -195,7 +195,7 @@ int nz_device_sm_count(int* sms);
 int nz_cells_count(const double* spheres64, int S, double Lx, double Ly, double Lz, int nx, int ny, int nz,
                    double jump_tol, int* counts, void* stream);
 
-/* Exclusive prefix sum of n ints (one block; n <= 1<<26); total receives the sum. */
+/* Exclusive prefix sum of n ints (n <= 1<<26); total receives the sum.  out may be in. */
 int nz_exclusive_scan_i32(const int* in, int* out, int n, int* total, void* stream);
 
 /* Member lists: items[offsets[c] ...] gets the counts[c] members of cell c in
@@ -240,12 +240,13 @@ int nz_cells_index(const int* items, int n_items, const int* perm, int S, const 
  * grown by 2 % of the reach, hold the (r + tol) balls with 2 nm and the
  * rounding of a half-precision distance to spare (margin: the near lists'
  * membership margin, which bounds the walker's distance and reach where the
- * near lists are taken).  After the pairs, a squared safe radius per record:
+ * near lists are taken).  Before the pairs, a squared safe radius per record:
  * a walker of the record's structure whose segment stays that close to the
  * record's centre meets no sphere.  idx, start, count: the near lists, laid
- * out without gaps (start the exclusive scan of count).  pack: nz_cells_pack_bytes(n_items, ncell, S) bytes, 16-byte
- * aligned; nz_substrate.near_items must then be n_items.  Grids with a cell
- * edge above 1e4 um and margins above 100 um are refused. */
+ * out without gaps (start the exclusive scan of count).  pack:
+ * nz_cells_pack_bytes(n_items, ncell, S) bytes, 16-byte aligned.  A substrate
+ * that names them as near_sph4 has the same S, grid and near_margin.  Grids
+ * with a cell edge above 1e4 um and margins above 100 um are refused. */
 size_t nz_cells_pack_bytes(int n_items, int ncell, int S);
 int nz_cells_pack(const float* rec4, const int* rec_sid, int S, const void* idx, int idx_bytes, const int* start,
                   const int* count, int n_items, const nz_grid* grid, float margin, void* pack, void* stream);

@@ -1221,7 +1221,7 @@ extern "C" int nz_cells_index(const int* items, int n_items, const int* perm, in
 
 extern "C" size_t nz_cells_pack_bytes(int n_items, int ncell, int S) {
   if (n_items < 0 || ncell < 0 || S < 0) return 0;
-  return pack_pairs(n_items, ncell) * 16 + size_t(S) * sizeof(float);
+  return (pack_radii(S) + pack_pairs(n_items, ncell)) * 16;
 }
 
 extern "C" int nz_cells_pack(const float* rec4, const int* rec_sid, int S, const void* idx, int idx_bytes,
@@ -1245,8 +1245,8 @@ extern "C" int nz_cells_pack(const float* rec4, const int* rec_sid, int S, const
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const unsigned blocks = unsigned((8 * ncell + 255) / 256);
   const float4* r = reinterpret_cast<const float4*>(rec4);
-  uint4* out = static_cast<uint4*>(pack);
-  float* safe = reinterpret_cast<float*>(out + pack_pairs(n_items, int(ncell)));
+  float* safe = static_cast<float*>(pack);
+  uint4* out = static_cast<uint4*>(pack) + pack_radii(S);
   const unsigned sblocks = unsigned((size_t(S) * 32 + 255) / 256);
   if (idx_bytes == 2)
     cells_pack_kernel<<<blocks, 256, 0, st>>>(r, static_cast<const uint16_t*>(idx), start, count, g, h, margin, out);

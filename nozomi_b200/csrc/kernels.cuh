@@ -65,6 +65,9 @@ constexpr size_t kSmemPerSm = 228 * 1024;  // shared memory an SM can give its C
 #define NZ_FUSED_MIN_BLOCKS 3
 #endif
 constexpr int kFusedMinBlocks = NZ_FUSED_MIN_BLOCKS;  // 256-thread CTAs per SM the register budget is sized for
+// A substrate's packed near entries (nz_cells_pack): the squared safe radius
+// of every record, up to a multiple of 16 bytes, then the pairs.
+__host__ __device__ inline size_t pack_radii(int S) { return (size_t(S) + 3) / 4; }  // in 16 bytes
 // Pairs of the packed near entries of n_items entries in ncell cells: the
 // pairs of cell c begin at (start[c] + c + 1) / 2; the walk may read a pair
 // past a cell's last one.

@@ -1212,11 +1212,10 @@ __host__ __device__ JobDev make_job(const nz_substrate& sub, const float* G, con
   j.near_start = sub.near_start;
   j.near_count = sub.near_count;
   j.near_sph4 = reinterpret_cast<const float4*>(sub.near_sph4);
-  // packed near entries: the pairs, then the squared safe radius of every record
-  j.near_pack = (sub.idx_bytes & NZ_NEAR_PACKED) && sub.near_idx ? reinterpret_cast<const uint4*>(sub.near_sph4)
-                                                                 : nullptr;
-  j.rec_safe = j.near_pack ? reinterpret_cast<const float*>(j.near_pack + pack_pairs(sub.near_items, j.ncell))
-                           : nullptr;
+  // packed near entries: the squared safe radius of every record, then the pairs
+  const bool packed = (sub.idx_bytes & NZ_NEAR_PACKED) && sub.near_idx && sub.near_sph4;
+  j.rec_safe = packed ? sub.near_sph4 : nullptr;
+  j.near_pack = packed ? reinterpret_cast<const uint4*>(sub.near_sph4) + pack_radii(sub.S) : nullptr;
   j.near_sid = sub.near_sid;
   j.idx = sub.idx_bytes ? sub.cell_idx : nullptr;
   j.near_idx = sub.idx_bytes ? sub.near_idx : nullptr;
