@@ -11,7 +11,12 @@ namespace nz {
 // the rounds of SimGeometry3D.gpu_seed (geometry.py:146-168) moved inside the
 // kernel and bounded.  The label of a point is found from its cell's list:
 // every sphere that contains a point of a cell is a member of that cell.
+// Bound by the latency of a round's loads, one after the other, where few
+// walkers need many rounds (2,000 in one axon of 60 over index lists: 3.1 ms an
+// entry at a time, 1.8 so, 2.5 over the arrays), else by the loads themselves.
 // ---------------------------------------------------------------------------
+constexpr int kAhead = 4;
+
 template <int LK>
 __global__ void seed_kernel(nz_substrate sub, const uint8_t* __restrict__ target, uint32_t id0, int N, uint32_t k0,
                             uint32_t k1, uint32_t stream, int max_rounds, float* __restrict__ spins,
@@ -35,16 +40,26 @@ __global__ void seed_kernel(nz_substrate sub, const uint8_t* __restrict__ target
     const int start = sub.cell_start[cell], count = sub.cell_count[cell];
     int lab = ns;
     if constexpr (LK != 0) {  // index lists: structures ascend, the first containing entry decides
-      for (int n = 0; n < count; ++n) {
-        const int key = LK == 2 ? int(static_cast<const unsigned short*>(sub.cell_idx)[start + n])
-                                : static_cast<const int*>(sub.cell_idx)[start + n];
-        const float4 c = __ldg(reinterpret_cast<const float4*>(sub.rec4) + key);
-        const float dx = px - c.x, dy = py - c.y, dz = pz - c.z;
-        if (dx * dx + dy * dy + dz * dz - c.w * c.w < 0) {
-          lab = sub.rec_sid[key];
-          break;
+      // kAhead entries at a time: their loads, two dependent ones each, in flight together
+      int found = -1;
+      for (int n = 0; n < count && found < 0; n += kAhead) {
+        int key[kAhead];
+        float4 c[kAhead];
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+          const int at = start + min(n + u, count - 1);
+          key[u] = LK == 2 ? int(__ldg(static_cast<const unsigned short*>(sub.cell_idx) + at))
+                           : __ldg(static_cast<const int*>(sub.cell_idx) + at);
+        }
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) c[u] = __ldg(reinterpret_cast<const float4*>(sub.rec4) + key[u]);
+#pragma unroll
+        for (int u = kAhead - 1; u >= 0; --u) {
+          const float dx = px - c[u].x, dy = py - c[u].y, dz = pz - c[u].z;
+          if (dx * dx + dy * dy + dz * dz - c[u].w * c[u].w < 0) found = key[u];
         }
       }
+      if (found >= 0) lab = __ldg(sub.rec_sid + found);
     }
     for (int n = 0; LK == 0 && n < count; ++n) {
       const int s = sub.cell_items[start + n];
@@ -347,7 +362,7 @@ extern "C" int nz_seed_range(const nz_substrate* sub, const uint8_t* target, uin
   if (N == 0) return NZ_OK;
   // index lists, where the substrate has them: a record an entry instead of
   // five arrays, and no entry past the first that contains the point (2e5
-  // walkers in axons on 20^3 cells: 0.33 ms against 0.45)
+  // walkers in axons on 20^3 cells: 0.33 ms against 0.45 an entry at a time)
   const int width = sub->cell_idx && sub->rec4 && sub->rec_sid && (reinterpret_cast<uintptr_t>(sub->rec4) & 15) == 0
                         ? sub->idx_bytes & ~NZ_NEAR_PACKED
                         : 0;
