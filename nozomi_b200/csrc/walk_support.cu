@@ -216,8 +216,11 @@ __device__ __forceinline__ double block_sum(double v, double* s_red) {
 // the sines' and cosines': 30 x 4 x 1e6 of them take 0.22 ms on a B200 (84 %
 // of the issue slots), 0.54 ms when every (direction, b) of 256 walkers was
 // summed over a block with two barriered reductions.
+// Where many threads share a pair their sums are folded first: one direction
+// and b of 1e5 walkers took 20 us with 384 sums added by one thread, 16.7 so.
 constexpr int kSigTile = 512;
 constexpr int kSigMaxThreads = 384;
+constexpr int kSigSerial = 8;  // groups whose sums one thread adds up
 
 __global__ void __launch_bounds__(kSigMaxThreads) signal_kernel(nz_state st, const float* __restrict__ dirs, int ndir,
                                                                 const float* __restrict__ amp, int nb, int combos,
@@ -259,6 +262,14 @@ __global__ void __launch_bounds__(kSigMaxThreads) signal_kernel(nz_state st, con
   s_sum[0][t] = re;
   s_sum[1][t] = im;
   __syncthreads();
+  for (; groups > kSigSerial; groups = (groups + 1) / 2) {  // few pairs: the upper half onto the lower
+    const int half = (groups + 1) / 2;
+    if (group + half < groups) {
+      s_sum[0][t] = re += s_sum[0][t + half * combos];
+      s_sum[1][t] = im += s_sum[1][t + half * combos];
+    }
+    __syncthreads();
+  }
   if (t < combos && combo < ndir * nb) {
     for (int g = 1; g < groups; ++g) {
       re += s_sum[0][t + g * combos];
