@@ -485,6 +485,11 @@ int nz_probe_fma(int grid, int iters, float* out, void* stream);
  * aligned. ---- */
 int nz_probe_box_muller(const uint32_t* words, int n, float* out, void* stream);
 
+/* ---- testing aid (no reference counterpart): *differ (one on the device) =
+ * how many of the 2^32 words give, on either side of the packed arithmetic, a
+ * quotient or a root in the draws' transform other than the IEEE operators'. ---- */
+int nz_probe_draw_operators(unsigned long long* differ, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

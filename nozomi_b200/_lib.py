@@ -127,6 +127,7 @@ SIGNATURES = {
     "nz_moments": (_i, [_P, _P, _i, _P, _P]),
     "nz_probe_fma": (_i, [_i, _i, _P, _P]),
     "nz_probe_box_muller": (_i, [_P, _i, _P, _P]),
+    "nz_probe_draw_operators": (_i, [_P, _P]),
 }
 
 _lib = None
