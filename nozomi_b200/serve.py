@@ -133,8 +133,8 @@ class Server:
         self.dev = dev
         self.compute = torch.cuda.current_stream(dev)
         self.side = torch.cuda.Stream(dev)
-        self.grids = {(lk, packed): batch_grid(threads, lk, self.tuning.stage, packed)
-                      for lk in (0, 2, 4) for packed in (False, True)}
+        near = self.tuning.near_margin is not None
+        self.grids = {(lk, bool(lk) and near): batch_grid(threads, lk, self.tuning.stage, near) for lk in (0, 2, 4)}
         self.queue = torch.zeros(3, dtype=torch.int32, device=dev)
         self.sort_scratch = torch.empty(1, dtype=torch.uint8, device=dev)
         self.clock = time.perf_counter
@@ -284,6 +284,8 @@ class Server:
                                       stream), "nz_batch_sort")
             self.queue.zero_()
             for g, (lk, packed, items) in enumerate(groups):
+                if (lk, packed) not in self.grids:  # near lists that could not be packed
+                    self.grids[lk, packed] = batch_grid(self.threads, lk, self.tuning.stage, packed)
                 launch_batch(table, len(jobs), items, lk, 0, k, self.queue.data_ptr() + 4 * g,
                              self.grids[lk, packed], self.threads, self.tuning.stage, stream, packed)
             e1.record(self.compute)
