@@ -13,24 +13,26 @@
 //    pass proves that label (some containing sphere of that structure, none of
 //    a lower one) or the iteration is redone with the recomputed label, so the
 //    result is the reference's;
-//  * a walker whose segment stays in the safe ball of the sphere that held it
-//    last (nz_cells_safe) takes its whole jump and scans nothing: three of
-//    four iterations of walkers inside axons;
-//  * the others scan their list in two passes.  The first marks the near
-//    spheres, those whose (r + tol) ball comes within 2 nm and 2 % of the
-//    reach of the segment ahead, from packed entries in half precision, two
-//    spheres an instruction; any other sphere neither contains the walker nor
-//    can lower the jump fraction.  The second runs the reference's inside
-//    test and the fractions for the marked ones only;
 //  * the near lists (the same cell grid with a smaller margin) serve every
-//    iteration whose reach fits their margin; the full lists the rest, scanned
-//    by the whole warp together;
+//    iteration whose reach fits their margin, the full lists the rest;
 //  * list entries are record indices (or, in record lists, carry their
-//    sphere's record and structure id inline); lists without packed entries
-//    are walked a lane a walker (walk_one);
+//    sphere's record and structure id inline);
+//  * packed near lists (nz_cells_pack) are walked by warps (walk_warp).  A
+//    walker whose segment stays in the safe ball of the sphere that held it
+//    last takes its whole jump and scans nothing: three of four iterations of
+//    walkers inside axons.  The others scan their list in two passes: the
+//    first marks the near spheres, those whose (r + tol) ball comes within
+//    2 nm and 2 % of the reach of the segment ahead, from the packed entries
+//    in half precision, two spheres an instruction; any other sphere neither
+//    contains the walker nor can lower the jump fraction.  The second runs
+//    the reference's inside test and the fractions for the marked ones only.
+//    Full lists are scanned by the whole warp together;
+//  * all other lists are walked by each lane on its own (walk_one), the near
+//    spheres marked by their distance from the walker against the reach;
 //  * each iteration has one draw site (the scatter draw of this step or the
 //    first draw of the next), and the inside and outside fractions share one
-//    instruction stream with one division (step_one);
+//    instruction stream (step_either; with one division, step_one, in
+//    walk_warp);
 //  * phase is accrued as the 3-vector Phi = sum_n G_n p_n with Kahan
 //    compensation, the wrap correction on the wrapped axis only; every
 //    direction's phase is u_d . Phi (the reference's per-direction sums
@@ -51,7 +53,7 @@ struct ScanOut {
 };
 
 // Dynamic shared memory: the records of a job (staged batched walk only),
-// then, in the phase modes, each thread's walker's Phi with its compensation
+// then, in walk_warp's phase modes, each thread's walker's Phi with its compensation
 // (a float4 per thread: Phi, compensation x; then a float2 per thread:
 // compensation y, z), or, in the moment modes, its origin (a float4 per
 // thread).  They are touched once a step and would hold registers through the
@@ -431,17 +433,18 @@ __device__ __forceinline__ void jump_of(const JobDev& J, uint32_t wid, int s, in
 // walker-steps on a packed substrate took 49.5 ms with every entry's record
 // filtered in single precision against the reach, and up to five fractions
 // for a warp's worst lane; 40.4 ms so.  Tried: all lanes' entries, or their
-// marked ones, pooled over the warp in shared memory (56.3, 48.5 ms).  Registers hold position, label, Phi and
-// its compensation and the step's jump; the origin (spins0) and the flag word
-// stay in memory and are updated in place on the rare wrap / iteration-cap
-// events (except with moments, which read the origin every step).
+// marked ones, pooled over the warp in shared memory (56.3, 48.5 ms).
+// Registers hold position, label and the step's jump, shared memory Phi and its
+// compensation; the origin (spins0) and the flag word stay in memory and are
+// updated in place on the rare wrap / iteration-cap events (with moments, which
+// read the origin every step, it is in shared memory too).
 template <int MODE, int LK, bool SH>
 __device__ __forceinline__ void walk_warp(const JobDev& J, bool live, int w, int s0, int s1,
                                           double* s_mom, float4* s_phi) {
   static_assert(LK != 0, "index lists only");
   constexpr bool kMom = (MODE & NZ_MODE_MOMENTS) != 0;
   constexpr bool kDisp = (MODE & kModeDisp) != 0;
-  constexpr bool kOrig = kMom || kDisp;  // origin in registers
+  constexpr bool kOrig = kMom || kDisp;  // origin in shared memory
   constexpr bool kT64 = (MODE & NZ_MODE_TANGENT64) != 0;
   constexpr unsigned kAll = 0xffffffffu;
   const int lane = threadIdx.x & 31;
@@ -467,7 +470,7 @@ __device__ __forceinline__ void walk_warp(const JobDev& J, bool live, int w, int
   float ds = 0.f;
   int oob = 0;  // bounds-checked build: an index was out of range
   int lo = 0, hi = 0;  // keys of structure `label`
-  int within = -1;     // index form: record of a sphere that contained the walker (-1: none known)
+  int within = -1;     // record of a sphere that contained the walker (-1: none known)
   const float dt = J.dt;
   const bool has_near = J.near_pack != nullptr;  // else the warp tests the full lists
   if (live) {
@@ -739,10 +742,11 @@ __device__ __forceinline__ void walk_warp(const JobDev& J, bool live, int w, int
 
 // Steps [s0, s1) of walker w, by a lane on its own: lists without packed
 // entries (on full lists of 25 entries, 1e8 walker-steps: 11.0 ms so, 11.7
-// through walk_warp, record lists 12.3 and 14.0).  Registers hold position, label, Phi and its
-// compensation and the step's jump; the origin (spins0) and the flag word stay
-// in memory and are updated in place on the rare wrap / iteration-cap events
-// (except with moments, which read the origin every step).
+// through walk_warp with single-precision marks, record lists 12.3 and 14.0).
+// Registers hold position, label, Phi and its compensation and the step's
+// jump; the origin (spins0) and the flag word stay in memory and are updated
+// in place on the rare wrap / iteration-cap events (except with moments, which
+// read the origin every step).
 template <int MODE, int LK, bool SH, bool BOX>
 __device__ __forceinline__ void walk_one(const JobDev& J, int w, int s0, int s1, double* s_mom) {
   constexpr bool kMom = (MODE & NZ_MODE_MOMENTS) != 0;
@@ -1011,9 +1015,9 @@ __device__ __forceinline__ void stage_records(uint32_t bar, const float4* src, u
 }
 
 // Work items are CTAs' worth of walkers of one job.  SINGLE: one job passed by
-// value, stage_cap walkers a warp, item i = the i-th CTA's worth of them.  Otherwise jobs and items come from
-// device arrays; with queue != null the grid is persistent and each CTA takes
-// items from *queue until none is left.
+// value, stage_cap walkers a warp, item i = the i-th CTA's worth of them.
+// Otherwise jobs and items come from device arrays; with queue != null the
+// grid is persistent and each CTA takes items from *queue until none is left.
 // STAGE (batched, index lists): a job whose S records fit in stage_cap
 // records is walked with its records in shared memory (s_stage, stage_cap *
 // 16 bytes of dynamic shared memory); the copy is made when a CTA's item
