@@ -115,6 +115,7 @@ struct JobDev {
   const void* near_idx;
   const uint4* near_pack;  // packed near entries (NZ_NEAR_PACKED), or null
   const float* rec_safe;   // with them: squared safe radius of each record
+  float pack_cut;          // near_cut with packed near entries, else -1
   const float4* rec4;
   const int* rec_sid;
   const int* sid_start;

@@ -55,13 +55,13 @@ struct ScanOut {
 // Dynamic shared memory: the records of a job (staged batched walk only),
 // then, in walk_warp's phase modes, each thread's walker's Phi with its compensation
 // (a float4 per thread: Phi, compensation x; then a float2 per thread:
-// compensation y, z), or, in the moment modes, its origin (a float4 per
-// thread).  They are touched once a step and would hold registers through the
-// collision pass.
+// compensation y, z), in its other modes its origin and id (a float4 per
+// thread; the origin in the moment modes only).  They are touched once a step
+// or draw and would hold registers through the collision pass.
 extern __shared__ __align__(16) float4 s_stage[];
 template <int MODE>
 constexpr size_t phi_bytes(int threads) {
-  return (MODE & NZ_MODE_PHI) ? size_t(threads) * 24 : (MODE & (NZ_MODE_MOMENTS | kModeDisp)) ? size_t(threads) * 16 : 0;
+  return size_t(threads) * ((MODE & NZ_MODE_PHI) ? 24 : 16);
 }
 
 // Record `key` of the substrate's record array (SH: the staged copy).  In
@@ -445,6 +445,7 @@ __device__ __forceinline__ void walk_warp(const JobDev& J, bool live, int w, int
   constexpr bool kMom = (MODE & NZ_MODE_MOMENTS) != 0;
   constexpr bool kDisp = (MODE & kModeDisp) != 0;
   constexpr bool kOrig = kMom || kDisp;  // origin in shared memory
+  constexpr bool kPhi = (MODE & NZ_MODE_PHI) != 0;
   constexpr bool kT64 = (MODE & NZ_MODE_TANGENT64) != 0;
   constexpr unsigned kAll = 0xffffffffu;
   const int lane = threadIdx.x & 31;
@@ -454,7 +455,7 @@ __device__ __forceinline__ void walk_warp(const JobDev& J, bool live, int w, int
   float sig = 1.f;
   static_assert(!(kOrig && (MODE & NZ_MODE_PHI)), "one of phase sums and origin");
   float4& phi_sum = s_phi[threadIdx.x];  // phase modes only
-  float4& origin = s_phi[threadIdx.x];   // moment modes only
+  float4& origin = s_phi[threadIdx.x];   // other modes: origin (moment modes) and id
   float2& phi_comp = reinterpret_cast<float2*>(s_phi + blockDim.x)[threadIdx.x];
   int s = live ? s0 : s1;
   int niter = 0, cell = 0;
@@ -472,7 +473,6 @@ __device__ __forceinline__ void walk_warp(const JobDev& J, bool live, int w, int
   int lo = 0, hi = 0;  // keys of structure `label`
   int within = -1;     // record of a sphere that contained the walker (-1: none known)
   const float dt = J.dt;
-  const bool has_near = J.near_pack != nullptr;  // else the warp tests the full lists
   if (live) {
     const float4 P = J.pos[w];
     x = P.x; y = P.y; z = P.z;
@@ -484,13 +484,13 @@ __device__ __forceinline__ void walk_warp(const JobDev& J, bool live, int w, int
       phi_sum = make_float4(F.x, F.y, F.z, C.x);
       phi_comp = make_float2(C.y, C.z);
     }
-    if (kOrig) origin = J.org[w];
+    if (!kPhi) origin = J.org[w];
     if (label < 0 || label > J.nstructures) label = J.nstructures;
     label_bounds<LK>(J, label, lo, hi);
     ds_label = label;
     ds = sqrtf(2 * __ldg(J.D + label) * dt);
     cell = step_cell(J, x, y, z, mx, my, mz);
-    cell_list(J, has_near, cell, pstart, pcount, oob);
+    cell_list(J, true, cell, pstart, pcount, oob);
     jump_of(J, wid, s, 0, ds, jx, jy, jz);
   }
   while (__any_sync(0xffffffffu, s < s1)) {
@@ -502,17 +502,14 @@ __device__ __forceinline__ void walk_warp(const JobDev& J, bool live, int w, int
     // margin of the step's cell: distance from the walker to the cell plus
     // the reach, with 2 % + 2 nm of slack against rounding
     // ((dist + reach) * 1.02 + tol + 2 nm <= margin, as dist^2 <= t^2 with
-    // t = near_cut - reach).
-    bool near = false;
-    if (has_near) {
-      const float ex = fmaxf(0.f, __fmaf_rn(-0.5f, J.g.dLx, fabsf(x - mx)));
-      const float ey = fmaxf(0.f, __fmaf_rn(-0.5f, J.g.dLy, fabsf(y - my)));
-      const float ez = fmaxf(0.f, __fmaf_rn(-0.5f, J.g.dLz, fabsf(z - mz)));
-      const float t = J.near_cut - reach;
-      near = t >= 0.f && __fmaf_rn(ex, ex, __fmaf_rn(ey, ey, ez * ez)) <= t * t;
-    }
+    // t = pack_cut - reach).
+    const float dist_x = fmaxf(0.f, __fmaf_rn(-0.5f, J.g.dLx, fabsf(x - mx)));
+    const float dist_y = fmaxf(0.f, __fmaf_rn(-0.5f, J.g.dLy, fabsf(y - my)));
+    const float dist_z = fmaxf(0.f, __fmaf_rn(-0.5f, J.g.dLz, fabsf(z - mz)));
+    const float t = J.pack_cut - reach;
+    const bool near = t >= 0.f && __fmaf_rn(dist_x, dist_x, __fmaf_rn(dist_y, dist_y, dist_z * dist_z)) <= t * t;
     int start = pstart, count = act ? pcount : 0;
-    if (act && has_near && !near) cell_list(J, false, cell, start, count, oob);
+    if (act && !near) cell_list(J, false, cell, start, count, oob);
     // A sphere of the walker's structure whose safe ball (nz_cells_safe)
     // contains the segment's ends, and so all of it: the walker stays inside
     // that sphere and out of reach of every lower structure's, so it keeps
@@ -719,9 +716,9 @@ __device__ __forceinline__ void walk_warp(const JobDev& J, bool live, int w, int
         ds_label = label;
       }
       cell = step_cell(J, x, y, z, mx, my, mz);
-      cell_list(J, has_near, cell, pstart, pcount, oob);
+      cell_list(J, true, cell, pstart, pcount, oob);
     }
-    if (s < s1) jump_of(J, wid, next_step, next_draw, ds, jx, jy, jz);
+    if (s < s1) jump_of(J, kPhi ? wid : __float_as_uint(origin.w), next_step, next_draw, ds, jx, jy, jz);
   }
   if (!live) return;
   J.pos[w] = make_float4(x, y, z, __int_as_float(label));
@@ -1220,6 +1217,10 @@ __host__ __device__ JobDev make_job(const nz_substrate& sub, const float* G, con
   const bool packed = (sub.idx_bytes & NZ_NEAR_PACKED) && sub.near_idx && sub.near_sph4;
   j.rec_safe = packed ? sub.near_sph4 : nullptr;
   j.near_pack = packed ? reinterpret_cast<const uint4*>(sub.near_sph4) + pack_radii(sub.S) : nullptr;
+  // without packed entries walk_warp takes the full lists always
+  j.pack_cut = packed ? j.near_cut : -1.0f;
+  if (!j.near_start) j.near_start = j.cell_start;
+  if (!j.near_count) j.near_count = j.cell_count;
   j.near_sid = sub.near_sid;
   j.idx = sub.idx_bytes ? sub.cell_idx : nullptr;
   j.near_idx = sub.idx_bytes ? sub.near_idx : nullptr;
@@ -1254,7 +1255,7 @@ __host__ __device__ JobDev make_job(const nz_substrate& sub, const float* G, con
 template <int MODE>
 constexpr int fused_carveout() {
   constexpr size_t need = kFusedMinBlocks * phi_bytes<MODE>(kFusedMaxThreads) + 2 * kFusedMinBlocks * 1400;
-  return phi_bytes<MODE>(32) ? int((100 * need + kSmemPerSm - 1) / kSmemPerSm) : 0;
+  return int((100 * need + kSmemPerSm - 1) / kSmemPerSm);
 }
 
 // Dynamic shared memory of the staged kernel for stage_cap records, after
