@@ -74,27 +74,27 @@ BATCH_WORKLOAD = ("batched mixed workload: {jobs} substrates of {a0}-{a1} beaded
 KERNEL_SOURCES = ("nozomi_b200/csrc/walk_fused.cu", "nozomi_b200/csrc/nz_common.cuh", "nozomi_b200/csrc/kernels.cuh",
                   "nozomi_b200/csrc/cells.cu", "nozomi_b200/engine.py")
 
-# Per workload, from one ncu capture of walk_fused_kernel (--set full,
-# --clock-control none) on a small case of that workload: warp instructions
+# Per workload, from one ncu capture of walk_fused_kernel (--clock-control
+# none) on a small case of that workload: warp instructions
 # executed (smsp__inst_executed.sum) and DRAM bytes (dram__bytes_read.sum +
 # dram__bytes_write.sum) of the captured launch, divided by the walker-steps
 # that launch ran; kernel_sha: the sources' hash at capture.
 PROFILED = {
-    "packed": {"kernel_sha": "aa15194f838fa36b", "warp_inst_per_walker_step": 40.990,
-               "dram_bytes_per_walker_step": 1.8011,
+    "packed": {"kernel_sha": "b43120bcd2c0a735", "warp_inst_per_walker_step": 38.976,
+               "dram_bytes_per_walker_step": 1.7825,
                "shape": {"cell": 0.5, "near_margin": 0.5, "coarsen": 8, "threads": 128, "lists": "index",
                          "near_shape": "round", "stage": 0},
                "capture": "walk_fused_kernel<PHI, idx16> launch 3 of `python bench.py --workload packed --walkers "
                           "1000000 --steps-per-launch 200 --steps 1 --warmup 1 --no-cpu-baseline --e2e-steps 0` "
-                          "(200,000,000 walker-steps): 8,198,067,851 warp instructions, 360.2 MB DRAM"},
-    "batched": {"kernel_sha": "aa15194f838fa36b", "warp_inst_per_walker_step": 32.993,
-                "dram_bytes_per_walker_step": 0.5611,
-                "shape": {"cell": 1.0, "near_margin": 0.5, "coarsen": 4, "threads": 256, "lists": "index",
+                          "(200,000,000 walker-steps): 7,795,194,810 warp instructions, 356.5 MB DRAM"},
+    "batched": {"kernel_sha": "b43120bcd2c0a735", "warp_inst_per_walker_step": 31.515,
+                "dram_bytes_per_walker_step": 0.5434,
+                "shape": {"cell": 1.0, "near_margin": 0.5, "coarsen": 4, "threads": 128, "lists": "index",
                           "near_shape": "round", "stage": 0},
                 "capture": "walk_fused_kernel<PHI, idx16> launch 2 of `python bench.py --walker-scale 0.1 --steps 1 "
                            "--warmup 1 --no-serving --no-plain --no-cpu-baseline --e2e-steps 0 --no-autotune --cell 1.0 "
-                           "--coarsen 4 --steps-per-launch 2000 --threads 256` (64 jobs, 2,407,477,000 walker-steps): "
-                           "79,430,203,761 warp instructions, 1350.7 MB DRAM"},
+                           "--coarsen 4 --steps-per-launch 2000 --threads 128` (64 jobs, 2,407,477,000 walker-steps): "
+                           "75,872,162,217 warp instructions, 1308.2 MB DRAM"},
 }
 
 

@@ -432,7 +432,7 @@ __device__ __forceinline__ void jump_of(const JobDev& J, uint32_t wid, int s, in
 // without the last spills are slower, 64 with more of them too): 8e8
 // walker-steps on a packed substrate took 49.5 ms with every entry's record
 // filtered in single precision against the reach, and up to five fractions
-// for a warp's worst lane; 40.4 ms so.  Tried: all lanes' entries, or their
+// for a warp's worst lane; 38.8 ms so.  Tried: all lanes' entries, or their
 // marked ones, pooled over the warp in shared memory (56.3, 48.5 ms).
 // Registers hold position, label and the step's jump, shared memory Phi and its
 // compensation; the origin (spins0) and the flag word stay in memory and are
