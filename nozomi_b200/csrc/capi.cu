@@ -3,6 +3,7 @@
 #include <cstdarg>
 #include <cstdint>
 #include <cstdio>
+#include <mutex>
 #include "kernels.cuh"
 
 namespace nz {
@@ -218,16 +219,99 @@ static int batch_list_kind(int mode) {
   return (mode & NZ_LIST_IDX16) ? 2 : (mode & NZ_LIST_IDX32) ? 4 : 0;
 }
 
+// Single-substrate walks that other streams of a device have not finished: an
+// event behind each stream's last one, for up to kSlots streams.  They only
+// decide how walkers are spread over warps (fused_lanes), never a result.  A
+// stream that is being captured is left out, as are all while the caller has
+// an error pending.
+class WalksInFlight {
+ public:
+  explicit WalksInFlight(cudaStream_t st) : st_(st) {
+    cudaStreamCaptureStatus status;
+    ok_ = cudaPeekAtLastError() == cudaSuccess && cudaGetDevice(&dev_) == cudaSuccess && dev_ >= 0 &&
+          dev_ < kMaxDevices && cudaStreamIsCapturing(st, &status) == cudaSuccess &&
+          status == cudaStreamCaptureStatusNone;
+    if (!ok_) return;
+    // another thread's capture is none of these calls' business
+    cudaThreadExchangeStreamCaptureMode(&mode_);
+  }
+  ~WalksInFlight() {
+    if (ok_) cudaThreadExchangeStreamCaptureMode(&mode_);
+  }
+  // Walkers in flight on other streams, counted up to `enough`.
+  long long walkers_elsewhere(long long enough) {
+    if (!ok_) return 0;
+    Device& d = devices()[dev_];
+    std::lock_guard<std::mutex> hold(d.m);
+    long long n = 0;
+    for (Slot& s : d.slots) {
+      if (n >= enough) break;
+      if (s.walkers == 0 || s.stream == st_) continue;
+      const cudaError_t e = cudaEventQuery(s.done);
+      if (e == cudaErrorNotReady) n += s.walkers;
+      else s.walkers = 0;
+      if (e != cudaSuccess) cudaGetLastError();
+    }
+    return n;
+  }
+  void launched(int walkers) {
+    if (!ok_) return;
+    Device& d = devices()[dev_];
+    std::lock_guard<std::mutex> hold(d.m);
+    Slot* at = nullptr;
+    for (Slot& s : d.slots) {
+      if (s.walkers && s.stream == st_) {
+        at = &s;
+        break;
+      }
+      if (!at && !s.walkers) at = &s;
+    }
+    if (!at) return;
+    at->walkers = 0;
+    at->stream = st_;
+    if ((!at->done && cudaEventCreateWithFlags(&at->done, cudaEventDisableTiming) != cudaSuccess) ||
+        cudaEventRecord(at->done, st_) != cudaSuccess)
+      cudaGetLastError();
+    else
+      at->walkers = walkers;
+  }
+
+ private:
+  static constexpr int kSlots = 32;
+  struct Slot {
+    cudaStream_t stream;
+    cudaEvent_t done;  // kept for the next launch that takes the slot
+    int walkers;       // 0: free
+  };
+  struct Device {
+    std::mutex m;
+    Slot slots[kSlots] = {};
+  };
+  static Device* devices() {
+    static Device d[kMaxDevices];
+    return d;
+  }
+  cudaStream_t st_;
+  int dev_ = 0;
+  bool ok_ = false;
+  cudaStreamCaptureMode mode_ = cudaStreamCaptureModeRelaxed;
+};
+
 // Walkers a warp of the single-substrate fused walk: 32, fewer for few
 // walkers.  A warp's step takes as long as its slowest lanes together, so
 // while warps are scarce, spreading the walkers over up to about two warps a
 // scheduler (1,250 on 148 SMs) shortens every step: 100 axons, 400 steps take
 // 1.92 ms for 2,003 walkers at 32 a warp, 1.73 / 1.47 / 1.30 / 1.25 / 1.36 at
 // 16 / 8 / 4 / 2 / 1; 5,000: 2.02, 1.79, 1.63, 1.57 at 4; 20,000: 2.12, 2.08
-// at 16, 2.22 at 8; 40,000: 2.52, 2.57 at 16.
-static int fused_lanes(int N) {
+// at 16, 2.22 at 8; 40,000: 2.52, 2.57 at 16.  Walkers in flight on other
+// streams count twice: their warps fill the schedulers already.  2,003 walkers
+// on each of 1 / 4 / 16 streams take 1.2 / 1.9 / 2.7 ms so, 1.2 / 2.4 / 6.9
+// by N alone and 2.3 / 2.4 / 3.0 at 32 a warp.
+static int fused_lanes(int N, WalksInFlight& flights) {
+  constexpr long long kWarps = 1250, kDense = 16 * kWarps;  // beyond kDense walkers: 32
+  const long long n = N > kDense ? N : N + 2 * flights.walkers_elsewhere((kDense - N) / 2 + 1);
   int lanes = 1;
-  while (lanes < 32 && N > lanes * 1250) lanes *= 2;
+  while (lanes < 32 && n > lanes * kWarps) lanes *= 2;
   return lanes;
 }
 
@@ -249,10 +333,13 @@ extern "C" int nz_walk_fused(const nz_substrate* sub, const nz_state* st, int mo
   if (step0 < 0 || step1 < step0) return set_error(NZ_ERR_ARG, "nz_walk_fused: bad step range");
   if (st->N == 0 || step1 == step0) return NZ_OK;
   const JobDev j = make_job(*sub, G, Garea, step1, dt, *draws, mode, *st, moments);
-  const int lanes = fused_lanes(st->N), per = kFusedThreads / 32 * lanes;
+  WalksInFlight flights(static_cast<cudaStream_t>(stream));
+  const int lanes = fused_lanes(st->N, flights), per = kFusedThreads / 32 * lanes;
   const int n_items = (st->N + per - 1) / per;
-  return launch_fused(mode, sub->idx_bytes & ~NZ_NEAR_PACKED, j, nullptr, nullptr, n_items, step0, step1, nullptr,
-                      n_items, kFusedThreads, static_cast<cudaStream_t>(stream), lanes);
+  rc = launch_fused(mode, sub->idx_bytes & ~NZ_NEAR_PACKED, j, nullptr, nullptr, n_items, step0, step1, nullptr,
+                    n_items, kFusedThreads, static_cast<cudaStream_t>(stream), lanes);
+  if (rc == NZ_OK) flights.launched(st->N);
+  return rc;
 }
 
 extern "C" size_t nz_walk_fused_moments_scratch_bytes(int N, int nsteps) {
@@ -280,11 +367,13 @@ extern "C" int nz_walk_fused_moments(const nz_substrate* sub, const nz_state* st
   const cudaStream_t cs = static_cast<cudaStream_t>(stream);
   JobDev j = make_job(*sub, G, Garea, step1, dt, *draws, mode, *st, nullptr);
   j.disp = scratch;
-  const int lanes = fused_lanes(st->N), per = kFusedThreads / 32 * lanes;
+  WalksInFlight flights(cs);
+  const int lanes = fused_lanes(st->N, flights), per = kFusedThreads / 32 * lanes;
   const int n_items = (st->N + per - 1) / per;
   rc = launch_fused(mode | kModeDisp, sub->idx_bytes & ~NZ_NEAR_PACKED, j, nullptr, nullptr, n_items, step0, step1,
                     nullptr, n_items, kFusedThreads, cs, lanes);
   if (rc) return rc;
+  flights.launched(st->N);
   const int gx = min(64, (st->N + 255) / 256);
   disp_moments_kernel<<<dim3(gx, step1 - step0), 256, 0, cs>>>(scratch, st->N, moments + size_t(step0) * 6);
   return check_launch("disp_moments_kernel");
