@@ -80,14 +80,14 @@ KERNEL_SOURCES = ("nozomi_b200/csrc/walk_fused.cu", "nozomi_b200/csrc/nz_common.
 # dram__bytes_write.sum) of the captured launch, divided by the walker-steps
 # that launch ran; kernel_sha: the sources' hash at capture.
 PROFILED = {
-    "packed": {"kernel_sha": "b43120bcd2c0a735", "warp_inst_per_walker_step": 38.976,
+    "packed": {"kernel_sha": "53355f7f88593302", "warp_inst_per_walker_step": 38.976,
                "dram_bytes_per_walker_step": 1.7825,
                "shape": {"cell": 0.5, "near_margin": 0.5, "coarsen": 8, "threads": 128, "lists": "index",
                          "near_shape": "round", "stage": 0},
                "capture": "walk_fused_kernel<PHI, idx16> launch 3 of `python bench.py --workload packed --walkers "
                           "1000000 --steps-per-launch 200 --steps 1 --warmup 1 --no-cpu-baseline --e2e-steps 0` "
                           "(200,000,000 walker-steps): 7,795,194,810 warp instructions, 356.5 MB DRAM"},
-    "batched": {"kernel_sha": "b43120bcd2c0a735", "warp_inst_per_walker_step": 31.515,
+    "batched": {"kernel_sha": "53355f7f88593302", "warp_inst_per_walker_step": 31.515,
                 "dram_bytes_per_walker_step": 0.5434,
                 "shape": {"cell": 1.0, "near_margin": 0.5, "coarsen": 4, "threads": 128, "lists": "index",
                           "near_shape": "round", "stage": 0},

@@ -167,8 +167,10 @@ class DeviceSubstrate:
 
     def _pack(self, start, count, idx, n, margin):
         """The packed near entries of index lists (nz_cells_pack); None for
-        cells, margins or lists too large for it."""
-        if max(self.grid.dLx, self.grid.dLy, self.grid.dLz) > 1e4 or margin > 100.0 or n + self.ncell >= 2 ** 31:
+        cells, margins or lists too large for it, and for margins that are 0
+        in single precision."""
+        if (max(self.grid.dLx, self.grid.dLy, self.grid.dLz) > 1e4 or not 0.0 < np.float32(margin) <= 100.0
+                or n + self.ncell >= 2 ** 31):
             return None
         lib = L.load()
         pack = torch.empty(int(lib.nz_cells_pack_bytes(n, self.ncell, self.S)), dtype=torch.uint8, device=_dev())

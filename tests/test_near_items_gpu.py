@@ -7,6 +7,18 @@ pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
 
 
+def test_margin_below_single_precision_builds():
+    """Such near lists stay unpacked, and the plain step walks beside them."""
+    from nozomi_b200 import engine
+    sph = np.array([[0.0], [0.0], [0.0], [1.0], [0.0]])
+    sub = engine.DeviceSubstrate(sph, 1, (4.0,) * 3, (4, 4, 4), np.full(2, 2.0), np.full(2, 80.0), near_margin=1e-46)
+    assert not sub.near_packed and sub.near is not None
+    x = torch.zeros((3, 10), device="cuda")
+    wk = engine.Walkers.with_counters(x, x.clone())
+    engine.walk_step(sub, wk, 0, 0.005, 0.0, 0.0, 0, engine.philox_draws(1))
+    assert (wk.label == 0).all()
+
+
 @pytest.mark.parametrize("S", [1, 2, 3, 4, 301])  # the radii end inside or on a 16-byte line
 def test_packed_lists_without_their_length(S):
     from nozomi_b200 import engine, _lib as L
